@@ -216,42 +216,49 @@ __global__ void __launch_bounds__( 32 * MG_WARPS ) k_mg_fill( const MgLevel *__r
     }
 }
 
-// the coarsest level: the dense inverse of A + mu 1 1^T (Gauss-Jordan in FP64), one warp per problem
-__global__ void __launch_bounds__( 32 ) k_mg_bottom_build( const MgLevel *__restrict__ lv ) {
+// the coarsest level: the dense inverse of A + mu 1 1^T (Gauss-Jordan in FP64), a block per problem with a thread per
+// entry of the 32 x 64 tableau.  A chain of 32 dependent pivots: one warp walking the rows of each took 174 us at 32 rows
+// (the whole hierarchy of 1,000 2D seeds: 253 us, with the tableau in parallel 188)
+constexpr int MGB = 1024;
+__global__ void __launch_bounds__( MGB ) k_mg_bottom_build( const MgLevel *__restrict__ lv ) {
     const MgLevel &M = lv[ blockIdx.x ];
-    const int n = M.n, lane = threadIdx.x;
+    const int n = M.n, t = threadIdx.x;
     __shared__ double A[ MG_BOTTOM ][ 2 * MG_BOTTOM ];
-    double mu = 0;
-    for ( int i = 0; i < n; ++i ) mu += M.dia[ i ];
+    __shared__ float sd[ MG_BOTTOM ];
+    if ( t < n ) sd[ t ] = M.dia[ t ];
+    __syncthreads();
+    double mu = 0, dmax = 0;
+    for ( int i = 0; i < n; ++i ) { mu += sd[ i ]; dmax = fmax( dmax, double( sd[ i ] ) ); }
     mu = mu / ( n * n );
-    for ( int i = 0; i < n; ++i )
-        for ( int j = lane; j < 2 * n; j += 32 ) A[ i ][ j ] = j < n ? ( i == j ? double( M.dia[ i ] ) : 0.0 ) + mu : ( j - n == i ? 1.0 : 0.0 );
-    __syncwarp();
-    for ( int i = 0; i < n; ++i )
-        for ( int e = M.rp[ i ]; e < M.rp[ i + 1 ]; ++e )
-            if ( lane == 0 ) A[ i ][ M.col[ e ] ] -= M.val[ e ];
-    __syncwarp();
-    double dmax = 0;
-    for ( int i = 0; i < n; ++i ) dmax = fmax( dmax, double( M.dia[ i ] ) );
     dmax = dmax > 0 ? dmax : 1.0;
+    for ( int k = t; k < n * 2 * MG_BOTTOM; k += MGB ) {
+        const int i = k / ( 2 * MG_BOTTOM ), j = k % ( 2 * MG_BOTTOM );
+        if ( j < 2 * n ) A[ i ][ j ] = j < n ? ( i == j ? double( sd[ i ] ) : 0.0 ) + mu : ( j - n == i ? 1.0 : 0.0 );
+    }
+    __syncthreads();
+    if ( t < n )
+        for ( int e = M.rp[ t ]; e < M.rp[ t + 1 ]; ++e ) A[ t ][ M.col[ e ] ] -= M.val[ e ];
     for ( int k = 0; k < n; ++k ) {
-        __syncwarp();
-        if ( lane == 0 && ! ( A[ k ][ k ] > 1e-12 * dmax ) ) A[ k ][ k ] += dmax;
-        __syncwarp();
+        __syncthreads();
         double piv = A[ k ][ k ];
-        __syncwarp();
-        for ( int j = lane; j < 2 * n; j += 32 ) A[ k ][ j ] /= piv;
-        __syncwarp();
-        for ( int i = 0; i < n; ++i ) {
-            if ( i == k ) continue;
-            double f = A[ i ][ k ];
-            __syncwarp();
-            for ( int j = lane; j < 2 * n; j += 32 ) A[ i ][ j ] -= f * A[ k ][ j ];
-            __syncwarp();
+        if ( ! ( piv > 1e-12 * dmax ) ) piv += dmax;
+        // row k over the pivot, then the others less their multiple of it: each thread's two entries from the values
+        // of before this pivot
+        double v[ 2 ];
+        for ( int h = 0; h < 2; ++h ) {
+            const int q = t + h * MGB, i = q / ( 2 * MG_BOTTOM ), j = q % ( 2 * MG_BOTTOM );
+            if ( i >= n || j >= 2 * n ) continue;
+            const double a = ( j == k ? piv : A[ k ][ j ] ) / piv;
+            v[ h ] = i == k ? a : A[ i ][ j ] - A[ i ][ k ] * a;
+        }
+        __syncthreads();
+        for ( int h = 0; h < 2; ++h ) {
+            const int q = t + h * MGB, i = q / ( 2 * MG_BOTTOM ), j = q % ( 2 * MG_BOTTOM );
+            if ( i < n && j < 2 * n ) A[ i ][ j ] = v[ h ];
         }
     }
-    for ( int i = 0; i < n; ++i )
-        for ( int j = lane; j < n; j += 32 ) M.inv[ i * n + j ] = float( A[ i ][ n + j ] );
+    __syncthreads();
+    for ( int q = t; q < n * n; q += MGB ) M.inv[ q ] = float( A[ q / n ][ n + q % n ] );
 }
 
 // ---- apply: one V(1,1) cycle --------------------------------------------------------------------------------------------
@@ -420,7 +427,7 @@ void launch_mg_coarsen( const Launch &L, const MgLevel *lv, int nprob, const Chu
 }
 void launch_mg_bottom_build( const Launch &L, const MgLevel *lv, int nprob ) {
     if ( nprob <= 0 ) return;
-    k_mg_bottom_build<<<nprob, 32, 0, L.stream>>>( lv );
+    k_mg_bottom_build<<<nprob, MGB, 0, L.stream>>>( lv );
     ++*L.launches;
 }
 void launch_mg_down( const Launch &L, const MgLevel *lv, const VecDev *vs, const Chunk *ch, int nch ) {
