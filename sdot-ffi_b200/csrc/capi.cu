@@ -497,15 +497,18 @@ int32_t sdot_linear_solve( sdot_context ctx, int64_t n, const int64_t *row_ptr, 
         if ( nnz >= ( 1ll << 31 ) ) throw Error( SDOT_ERR_ARGS, "nnz must fit int32" );
         std::vector<int> rp32( hrp.begin(), hrp.end() );
         const long nch = ( n + vec_chunk( n ) - 1 ) / vec_chunk( n );
-        size_t bytes = size_t( n + 1 ) * 4 + size_t( nnz + 1 ) * 12 + size_t( n ) * 8 * 9 + size_t( nch ) * 32 + NB_SC * 8 + 64 + 16 * 256;
+        size_t bytes = size_t( n + 1 ) * 4 + size_t( nnz + 1 ) * 12 + size_t( n ) * 8 * 9 + size_t( nch ) * 32 + NB_SC * 8 + 64 + 17 * 256;
+        bytes += 2 * PCG_MAX_BLOCKS * sizeof( double2 );      // the team CG's sums
         if ( mixed ) bytes += size_t( nnz + 1 ) * 4 + size_t( n ) * 4 * 6 + 8 * 256;
         DevVec mem( c, bytes );
         Arena A{ ( char * ) mem.p, bytes, 0 };
         int *rp = A.take<int>( n + 1 ), *col = A.take<int>( nnz + 1 );
         double *val = A.take<double>( nnz + 1 ), *ddia = A.take<double>( n );
         double *xx = A.take<double>( n ), *r = A.take<double>( n ), *z = A.take<double>( n ), *p = A.take<double>( n ), *q = A.take<double>( n );
+        A.take<double>( n );                               // (z, p and q, this: the team CG's pairs)
         double *b = A.take<double>( n ), *d = A.take<double>( n ), *part = A.take<double>( size_t( nch ) * 4 ), *sc = A.take<double>( NB_SC );
         unsigned *counter = A.take<unsigned>( 2 );
+        double2 *part2 = A.take<double2>( 2 * PCG_MAX_BLOCKS );
         float *m32[ 7 ] = {};
         if ( mixed ) {
             m32[ 0 ] = A.take<float>( nnz + 1 );
@@ -557,13 +560,29 @@ int32_t sdot_linear_solve( sdot_context ctx, int64_t n, const int64_t *row_ptr, 
         V.tol = tol > 0 ? tol : 1e-10;
         V.maxit = maxit > 0 ? maxit : 100000;
         V.sc = sc; V.partials = part; V.counter = counter; V.nchunk = int( vch.size() ); V.active = 1;
+        if ( ! mixed ) {
+            V.pz = reinterpret_cast<double2 *>( z );
+            V.rq = reinterpret_cast<double2 *>( q );
+            V.part2 = part2;
+            V.p2 = d;
+        }
         V.rank0 = mg ? iperm[ 0 ] : 0;                     // the gauge x[ 0 ] = 0, row 0 wherever it went
         if ( mixed ) {
             V.mixed = 1;
             V.val32 = m32[ 0 ]; V.dia32 = m32[ 1 ]; V.x32 = m32[ 2 ]; V.r32 = m32[ 3 ]; V.z32 = m32[ 4 ]; V.p32 = m32[ 5 ]; V.q32 = m32[ 6 ];
         }
         size_t o1 = ( sizeof( VecDev ) + 255 ) & ~size_t( 255 );
-        DevVec dd( c, o1 + vch.size() * sizeof( Chunk ) );
+        // the team CG's launch: its problem (without a hierarchy), its blocks, its barrier
+        const PcgProb one{ 0, 0, 0 };
+        std::vector<int4> teams;
+        const int cluster = pcg_teams( std::vector<int>( 1, int( n ) ), teams );
+        const size_t o2 = o1 + ( ( vch.size() * sizeof( Chunk ) + 255 ) & ~size_t( 255 ) ), o3 = o2 + 256;
+        DevVec dd( c, o3 + teams.size() * sizeof( int4 ) );
+        PcgProb *dprob = reinterpret_cast<PcgProb *>( ( char * ) dd.p + o2 );
+        unsigned *dbar = reinterpret_cast<unsigned *>( ( char * ) dd.p + o2 + 128 );
+        int4 *dteams = reinterpret_cast<int4 *>( ( char * ) dd.p + o3 );
+        CK( cudaMemcpyAsync( dprob, &one, sizeof( one ), cudaMemcpyHostToDevice, c.stream ) );
+        CK( cudaMemcpyAsync( dteams, teams.data(), teams.size() * sizeof( int4 ), cudaMemcpyHostToDevice, c.stream ) );
         CK( cudaMemcpyAsync( dd.p, &V, sizeof( V ), cudaMemcpyHostToDevice, c.stream ) );
         CK( cudaMemcpyAsync( ( char * ) dd.p + o1, vch.data(), vch.size() * sizeof( Chunk ), cudaMemcpyHostToDevice, c.stream ) );
         VecDev *dv = dd.as<VecDev>();
@@ -585,6 +604,7 @@ int32_t sdot_linear_solve( sdot_context ctx, int64_t n, const int64_t *row_ptr, 
             CK( cudaMemcpyAsync( b, hb.data(), n * 8, cudaMemcpyHostToDevice, c.stream ) );
             double hsc[ NB_SC ] = {};
             hsc[ SC_MEAN ] = mean;
+            hsc[ SC_ITER ] = -1;
             CK( cudaMemcpyAsync( sc, hsc, sizeof( hsc ), cudaMemcpyHostToDevice, c.stream ) );
             if ( mg ) {
                 const int its = mg_linear_solve( c, V, nnz, hsc );
@@ -597,12 +617,10 @@ int32_t sdot_linear_solve( sdot_context ctx, int64_t n, const int64_t *row_ptr, 
                 continue;
             }
             if ( mixed ) launch_mx_init( L, dv, dch, int( vch.size() ) );
-            else launch_cg_init( L, dv, dch, int( vch.size() ) );
             for ( ;; ) {
-                for ( int s = 0; s < 32; ++s ) {
-                    if ( mixed ) launch_mx_iter( L, dv, dch, int( vch.size() ) );
-                    else launch_cg_iter( L, dv, dch, int( vch.size() ) );
-                }
+                if ( mixed )
+                    for ( int s = 0; s < 32; ++s ) launch_mx_iter( L, dv, dch, int( vch.size() ) );
+                else CK( launch_pcg( L, dprob, dteams, int( teams.size() ), cluster, 1, nullptr, dv, 256, dbar ) );
                 CK( cudaMemcpyAsync( hsc, sc, sizeof( hsc ), cudaMemcpyDeviceToHost, c.stream ) );
                 CK( cudaStreamSynchronize( c.stream ) );
                 if ( hsc[ SC_CONV ] != 0 ) break;

@@ -512,6 +512,7 @@ struct SolveJob {
     char *mg_mem = nullptr;
     int *row_ptr, *col, *rowcnt;
     double *part_cells, *part_vec;
+    double2 *part_pcg = nullptr;
     unsigned long long *wslot;          // [2]
     int wcur = 0;                       // wslot[ wcur ] belongs to w
     double *obary = nullptr, *ocost = nullptr;
@@ -587,7 +588,7 @@ size_t job_bytes( int dim, long n, int dkind, long dcount ) {
     b += size_t( n ) * ( dim == 2 ? 64 : 84 ) + 1024;    // the weight majorants and their moments (4/3, 8/7 of the grid's cells)
     b += dkind == D_IMAGE ? size_t( dcount ) * 32 + 32768 : size_t( dcount ) * 8 * ( dim + 2 );     // (image: values, prefix, original, blur pass)
     b += size_t( n ) * ( 24 + dim * 8 ) + 4096;
-    return b + mg_bytes( dim, n, cap );
+    return b + 2 * PCG_MAX_BLOCKS * sizeof( double2 ) + mg_bytes( dim, n, cap );
 }
 
 static void alloc_job( Ctx &c, SolveJob &J ) {
@@ -598,14 +599,15 @@ static void alloc_job( Ctx &c, SolveJob &J ) {
     J.ovf_cap = int( n ) + 4096;
     size_t bytes = size_t( n ) * 8 * 18 + 2 * ( size_t( n ) * 4 + size_t( n ) * cap * 12 ) + size_t( n + 1 ) * 4 + size_t( n ) * cap * 12 +
                    size_t( n ) * 4 + size_t( J.nch_cells ) * NB_REPORT * 8 + size_t( J.nch_vec ) * 4 * 8 + 64 + size_t( n ) * 8 * ( dim + 1 ) +
-                   2 * ( size_t( J.ovf_cap ) * 12 + 16 ) + ( J.agg_margin > 0 ? AGG_CAP * sizeof( int2 ) : 0 ) + 49 * 256;
+                   2 * ( size_t( J.ovf_cap ) * 12 + 16 ) + ( J.agg_margin > 0 ? AGG_CAP * sizeof( int2 ) : 0 ) + 2 * PCG_MAX_BLOCKS * sizeof( double2 ) + 50 * 256;
     J.mem_bytes = bytes;
     J.mem = ( char * ) dalloc( c, bytes );
     Arena A{ J.mem, bytes, 0 };
     J.w = A.take<double>( n ); J.w2 = A.take<double>( n ); J.a = A.take<double>( n ); J.a2 = A.take<double>( n );
     J.d = A.take<double>( n ); J.nu = A.take<double>( n ); J.nu_dev_user = A.take<double>( n ); J.b = A.take<double>( n );
     J.x = A.take<double>( n ); J.r = A.take<double>( n ); J.z = A.take<double>( n ); J.p = A.take<double>( n );
-    J.q = A.take<double>( n ); J.dia = A.take<double>( n ); J.tmpw = A.take<double>( n );
+    J.q = A.take<double>( n ); J.tmpw = A.take<double>( n ); J.dia = A.take<double>( n );       // (z, p and q, tmpw: the team CG's pairs)
+    J.part_pcg = A.take<double2>( 2 * PCG_MAX_BLOCKS );
     for ( int k = 0; k < 2; ++k ) {
         J.nb[ k ] = A.take<int>( n ); J.nid[ k ] = A.take<int>( size_t( n ) * cap ); J.nc[ k ] = A.take<double>( size_t( n ) * cap );
         J.ovf_count[ k ] = A.take<int>( 4 ); J.ovf_ids[ k ] = A.take<int>( J.ovf_cap ); J.ovf_c[ k ] = A.take<double>( J.ovf_cap );
@@ -1460,6 +1462,12 @@ static VecDev vec_of( Ctx &c, SolveJob &J ) {
         V.mixed = 1;
         V.val32 = J.val32; V.dia32 = J.dia32; V.x32 = J.x32; V.r32 = J.r32; V.z32 = J.z32; V.p32 = J.p32; V.q32 = J.q32;
     }
+    if ( ! V.mixed ) {
+        V.pz = reinterpret_cast<double2 *>( J.z );
+        V.rq = reinterpret_cast<double2 *>( J.q );
+        V.part2 = J.part_pcg;
+        V.p2 = J.d;                                   // (the direction is written once the CG has converged)
+    }
     if ( J.agg_margin > 0 ) {
         V.agg_pairs = J.agg_pairs;
         V.agg_cap = AGG_CAP;
@@ -1495,6 +1503,17 @@ struct VecBatch {
     int2 *dfidx = nullptr;
     Chunk *dbuild0 = nullptr;
     Chunk *ddown[ MG_MAX_LEVELS ], *dup[ MG_MAX_LEVELS ], *dcrs[ MG_MAX_LEVELS ];
+    // a batch of the team CG: every problem, and the levels of its hierarchy in one row
+    std::vector<PcgProb> cprob;
+    std::vector<MgLevel> cchain;
+    std::vector<int> crows;
+    struct Group { int prob, nprob, block, nblock, cluster; };     // the launches: at most PCG_MAX_BLOCKS problems each
+    std::vector<Group> groups;
+    std::vector<int4> cteams;
+    PcgProb *dcprob = nullptr;
+    int4 *dcteams = nullptr;
+    unsigned *dcbars = nullptr;
+    MgLevel *dcchain = nullptr;
 
     void add( const VecDev &d, const SolveJob *J = nullptr ) {
         int p = int( v.size() );
@@ -1505,7 +1524,13 @@ struct VecBatch {
         int k = 0;
         const int vc = vec_chunk( d.n );
         for ( int b = 0; b < d.n; b += vc, ++k ) ch.push_back( Chunk{ p, b, std::min( d.n, b + vc ), k } );
-        if ( ! J || ! J->mg_L || ! d.precond ) return;
+        const bool levels = J && J->mg_L && d.precond;
+        if ( J && d.pz ) {
+            cprob.push_back( PcgProb{ p, int( cchain.size() ), levels ? J->mg_L : 0 } );
+            for ( int l = 0; levels && l < J->mg_L; ++l ) cchain.push_back( mg_level( *J, l, p ) );
+            crows.push_back( d.n );
+        }
+        if ( ! levels ) return;
         maxL = std::max( maxL, J->mg_L );
         MgJob mj{ J, {} };
         for ( int l = 0; l < J->mg_L; ++l ) {
@@ -1580,6 +1605,20 @@ struct VecBatch {
         parts.push_back( { fchain.data(), fchain.size() * sizeof( MgLevel ) } );
         parts.push_back( { fidx.data(), fidx.size() * sizeof( int2 ) } );
         parts.push_back( { build0.data(), build0.size() * sizeof( Chunk ) } );
+        parts.push_back( { cprob.data(), cprob.size() * sizeof( PcgProb ) } );
+        parts.push_back( { cchain.data(), cchain.size() * sizeof( MgLevel ) } );
+        groups.clear();
+        cteams.clear();
+        for ( int b = 0; b < int( crows.size() ); b += PCG_MAX_BLOCKS ) {
+            const int e = std::min( int( crows.size() ), b + PCG_MAX_BLOCKS );
+            std::vector<int4> t;
+            const int cl = pcg_teams( std::vector<int>( crows.begin() + b, crows.begin() + e ), t );
+            groups.push_back( Group{ b, e - b, int( cteams.size() ), int( t.size() ), cl } );
+            cteams.insert( cteams.end(), t.begin(), t.end() );
+        }
+        const std::vector<unsigned> bars( crows.size(), 0u );
+        parts.push_back( { cteams.data(), cteams.size() * sizeof( int4 ) } );
+        parts.push_back( { bars.data(), bars.size() * sizeof( unsigned ) } );
         std::vector<size_t> off;
         size_t total = 0;
         for ( auto &p : parts ) { off.push_back( total ); total += ( p.second + 255 ) & ~size_t( 255 ); }
@@ -1599,6 +1638,10 @@ struct VecBatch {
         dfchain = reinterpret_cast<MgLevel *>( d + off[ k++ ] );
         dfidx = reinterpret_cast<int2 *>( d + off[ k++ ] );
         dbuild0 = reinterpret_cast<Chunk *>( d + off[ k++ ] );
+        dcprob = reinterpret_cast<PcgProb *>( d + off[ k++ ] );
+        dcchain = reinterpret_cast<MgLevel *>( d + off[ k++ ] );
+        dcteams = reinterpret_cast<int4 *>( d + off[ k++ ] );
+        dcbars = reinterpret_cast<unsigned *>( d + off[ k++ ] );
     }
     // the hierarchies of every job, from their fresh Laplacians
     void build( const Launch &L, ErrRec *err ) {
@@ -1608,6 +1651,11 @@ struct VecBatch {
         launch_mg_level0( L, dlv[ 0 ], dv, dbuild0, int( build0.size() ) );
         for ( int l = 0; l + 1 < maxL; ++l ) launch_mg_coarsen( L, dlv[ l ], int( lv[ l ].size() ), dcrs[ l ], int( crs[ l ].size() ), err );
         launch_mg_bottom_build( L, dbottom, int( bottom.size() ) );
+    }
+    // up to `burst` iterations of a batch of the team CG
+    void pcg( const Launch &L, int burst ) {
+        for ( const Group &g : groups )
+            CK( launch_pcg( L, dcprob + g.prob, dcteams + g.block, g.nblock, g.cluster, g.nprob, dcchain, dv, burst, dcbars + g.prob ) );
     }
     // z = M^-1 r for every job
     void vcycle( const Launch &L ) {
@@ -1660,6 +1708,7 @@ static void run_burst( Ctx &c, const std::vector<long long> &key, Issue issue ) 
 }
 
 constexpr int MG_BURST_SOLVE = 8;
+constexpr int PCG_BURST = 256;       // iterations of a team CG launch that nothing else waits for (a few ms)
 int mg_linear_solve( Ctx &c, const VecDev &V0, long nnz, double *hsc ) {
     SolveJob J;                                      // only its hierarchy is used
     J.G.dim = nnz > 10 * long( V0.n ) ? 3 : 2;       // the aggregates of a 3D Laplacian (about 15 entries a row) pack 8 rows
@@ -1681,29 +1730,23 @@ int mg_linear_solve( Ctx &c, const VecDev &V0, long nnz, double *hsc ) {
     Launch L = c.L();
     const int nch = int( B.ch.size() );
     const bool mixed = V.mixed != 0;
-    if ( B.mg() ) {
-        B.build( L, c.derr );
-        if ( mixed ) launch_mx_init( L, B.dv, B.dch, nch );
-        else launch_cg_init0( L, B.dv, B.dch, nch );
-        B.vcycle( L );
-        if ( mixed ) launch_mx_init1( L, B.dv, B.dch, nch );
-        else launch_cg_init1( L, B.dv, B.dch, nch );
-    } else if ( mixed )
+    if ( B.mg() ) B.build( L, c.derr );
+    if ( mixed ) {                                   // (the FP64 team CG starts by itself)
         launch_mx_init( L, B.dv, B.dch, nch );
-    else
-        launch_cg_init( L, B.dv, B.dch, nch );
+        if ( B.mg() ) {
+            B.vcycle( L );
+            launch_mx_init1( L, B.dv, B.dch, nch );
+        }
+    }
     for ( ;; ) {
-        for ( int k = 0; k < MG_BURST_SOLVE; ++k ) {
+        if ( ! mixed ) B.pcg( L, PCG_BURST );
+        else for ( int k = 0; k < MG_BURST_SOLVE; ++k ) {
             if ( B.mg() ) {
-                if ( mixed ) launch_mx_spmv_update( L, B.dv, B.dch, nch );
-                else launch_cg_spmv_update( L, B.dv, B.dch, nch );
+                launch_mx_spmv_update( L, B.dv, B.dch, nch );
                 B.vcycle( L );
-                if ( mixed ) launch_mx_rz_p( L, B.dv, B.dch, nch );
-                else launch_cg_rz_p( L, B.dv, B.dch, nch );
-            } else if ( mixed )
+                launch_mx_rz_p( L, B.dv, B.dch, nch );
+            } else
                 launch_mx_iter( L, B.dv, B.dch, nch );
-            else
-                launch_cg_iter( L, B.dv, B.dch, nch );
         }
         CK( cudaMemcpyAsync( hsc, V.sc, NB_SC * sizeof( double ), cudaMemcpyDeviceToHost, c.stream ) );
         CK( cudaMemcpyAsync( c.herr, c.derr, sizeof( ErrRec ), cudaMemcpyDeviceToHost, c.stream ) );
@@ -1742,13 +1785,13 @@ static void launch_pending( Ctx &c, std::vector<SolveJob *> &jobs ) {
         }
     }
     if ( ! newton.v.empty() ) {
-        // Jacobi- and multigrid-preconditioned problems, FP64 and mixed CG, go in four batches
-        VecBatch jac, mgb, jacx, mgbx;
+        // the FP64 systems in one batch, the Jacobi- and multigrid-preconditioned mixed ones in two
+        VecBatch team, jacx, mgbx;
         for ( size_t k = 0; k < newton.v.size(); ++k ) {
             const VecDev &v = newton.v[ k ];
-            ( v.precond ? ( v.mixed ? mgbx : mgb ) : ( v.mixed ? jacx : jac ) ).add( v, newton.jobs[ k ] );
+            ( ! v.mixed ? team : v.precond ? mgbx : jacx ).add( v, newton.jobs[ k ] );
         }
-        for ( VecBatch *B : { &jac, &mgb, &jacx, &mgbx } ) {
+        for ( VecBatch *B : { &jacx, &mgbx, &team } ) {
             if ( B->v.empty() ) continue;
             B->upload( c );
             const int nch = int( B->ch.size() );
@@ -1765,20 +1808,17 @@ static void launch_pending( Ctx &c, std::vector<SolveJob *> &jobs ) {
                 if ( J && J->ncl > 0 && J->cl_true )
                     launch_agg_cap( L, J->row_ptr, J->col, J->val, J->dia, J->d_cl, J->ncl, 1e6 * J->c_scale, J->cl_true );
             launch_rhs( L, B->dv, B->dch, nch );
-            const bool mixed = B == &jacx || B == &mgbx;
             if ( B->mg() ) {
                 c.timer.end( c.stream, 5 );
                 c.timer.begin( c.stream, K_MULTIGRID, rows );
                 B->build( L, c.derr );
-                if ( mixed ) launch_mx_init( L, B->dv, B->dch, nch );
-                else launch_cg_init0( L, B->dv, B->dch, nch );
+            }
+            // (the team CG starts by itself, in the next tick's burst)
+            if ( B != &team ) launch_mx_init( L, B->dv, B->dch, nch );
+            if ( B == &mgbx ) {
                 B->vcycle( L );
-                if ( mixed ) launch_mx_init1( L, B->dv, B->dch, nch );
-                else launch_cg_init1( L, B->dv, B->dch, nch );
-            } else if ( mixed )
-                launch_mx_init( L, B->dv, B->dch, nch );
-            else
-                launch_cg_init( L, B->dv, B->dch, nch );
+                launch_mx_init1( L, B->dv, B->dch, nch );
+            }
             c.timer.end( c.stream, 5 );
         }
     }
@@ -2003,15 +2043,24 @@ void jobs_tick( Ctx &c, std::vector<SolveJob *> &jobs ) {
         }
     }
     // B. CG iterations
-    VecBatch cgj, cgm, cgjx, cgmx;
+    VecBatch cgjx, cgmx, cgc;
     std::vector<SolveJob *> with_cg;
     for ( SolveJob *J : jobs )
         if ( J->state == J_CG ) {
             VecDev V = vec_of( c, *J );
-            ( V.precond ? ( V.mixed ? cgmx : cgm ) : ( V.mixed ? cgjx : cgj ) ).add( V, J );
+            ( ! V.mixed ? cgc : V.precond ? cgmx : cgjx ).add( V, J );
             with_cg.push_back( J );
         }
-    for ( VecBatch *B : { &cgj, &cgm, &cgjx, &cgmx } ) {
+    if ( ! cgc.v.empty() ) {
+        cgc.upload( c );
+        double rows = 0;
+        for ( auto &v : cgc.v ) rows += v.n;
+        c.timer.begin( c.stream, K_CG, rows );
+        // the launch ends with the iteration that converges; in a batch it does not hold the others' diagrams up for long
+        cgc.pcg( L, jobs.size() == 1 ? PCG_BURST : ( with_diag.empty() ? PCG_BURST / 4 : PCG_BURST / 8 ) );
+        c.timer.end( c.stream, 1 );
+    }
+    for ( VecBatch *B : { &cgjx, &cgmx } ) {
         if ( B->v.empty() ) continue;
         B->upload( c );
         const int nch = int( B->ch.size() );
@@ -2019,19 +2068,14 @@ void jobs_tick( Ctx &c, std::vector<SolveJob *> &jobs ) {
         if ( with_diag.empty() ) burst *= 4;
         double rows = 0;
         for ( auto &v : B->v ) rows += v.n;
-        const bool mixed = B == &cgjx || B == &cgmx;
         auto issue = [&]() {
             for ( int k = 0; k < burst; ++k ) {
                 if ( B->mg() ) {
-                    if ( mixed ) launch_mx_spmv_update( L, B->dv, B->dch, nch );
-                    else launch_cg_spmv_update( L, B->dv, B->dch, nch );
+                    launch_mx_spmv_update( L, B->dv, B->dch, nch );
                     B->vcycle( L );
-                    if ( mixed ) launch_mx_rz_p( L, B->dv, B->dch, nch );
-                    else launch_cg_rz_p( L, B->dv, B->dch, nch );
-                } else if ( mixed )
+                    launch_mx_rz_p( L, B->dv, B->dch, nch );
+                } else
                     launch_mx_iter( L, B->dv, B->dch, nch );
-                else
-                    launch_cg_iter( L, B->dv, B->dch, nch );
             }
         };
         unsigned long long l0 = c.launches;

@@ -15,6 +15,7 @@
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
+#include <vector>
 
 #define SDOT_DEV __device__ __forceinline__
 
@@ -176,6 +177,10 @@ struct VecDev {
     int maxit;                    // CG iterations at most
     const double *report;         // the Newton report of the accepted diagram (rhs)
     unsigned long long *wmax_slot;   // ordered-integer max of the trial weights
+    // the team CG (pcg.cu; NULL: this system takes the launches of linalg.cu): the pairs { z, p } (over z and p, which
+    // are contiguous) and { r, q } (over q and the vector after it), the direction p, the shares' sums [ 2 ][ PCG_MAX_BLOCKS ]
+    double2 *pz, *rq, *part2;
+    double *p2;
     double *sc;                   // [NB_SC] scalars of the problem
     double *partials;             // [nchunk * 4]
     unsigned *counter;
@@ -211,6 +216,11 @@ struct MgLevel {
     int capn;                          // entries the next level's col / val can hold
     float *inv;                        // the coarsest level: dense inverse [n * n]
 };
+
+// a problem of a team CG launch: its VecDev, and its multigrid levels chain[ first .. first + count ) (count 0: Jacobi)
+struct PcgProb { int vec, first, count; };
+constexpr int PCG_SHARE = 128;         // rows one block of a CG team works on, at least (pcg.cu)
+constexpr int PCG_MAX_BLOCKS = 148;    // blocks of a launch, and problems
 
 enum Scalar : int { SC_RZ = 0, SC_ALPHA, SC_BETA, SC_BNORM, SC_RNORM, SC_CONV, SC_ITER, SC_MEAN, SC_C, SC_TOL, SC_PQ, SC_FAIL, SC_NNZ,
                     SC_REFINE,      // mixed CG: 1 once the inner FP32 CG has converged (x += e, then the FP64 residual)
@@ -416,18 +426,19 @@ void launch_agg_direction( const Launch &L, const int *row_ptr, const int *col, 
                            const double *nu, const double *b, double *x, double *y );
 // the cluster shares of the masses: ae[ i ] = nu[ i ] a_C / nu_C for the members i of each cluster C (others untouched)
 void launch_agg_shares( const Launch &L, const double *a, const double *nu, const int *cl_begin, const int *cl_members, int ncl, double *ae );
-// the multigrid-preconditioned CG: init in two halves around the first V-cycle, then per iteration
-// spmv -> update -> V-cycle -> r.z -> p
-void launch_cg_init0( const Launch &L, const VecDev *v, const Chunk *ch, int nch );
-void launch_cg_init1( const Launch &L, const VecDev *v, const Chunk *ch, int nch );
-void launch_cg_spmv_update( const Launch &L, const VecDev *v, const Chunk *ch, int nch );
-void launch_cg_rz_p( const Launch &L, const VecDev *v, const Chunk *ch, int nch );
-// the mixed CG (FP32 inner CG, FP64 iterative refinement): the same sequence of launches as the FP64 CG
+// the mixed CG (FP32 inner CG, FP64 iterative refinement); with the multigrid: init in two halves around the first V-cycle,
+// then per iteration spmv -> update -> V-cycle -> r.z -> p
 void launch_mx_init( const Launch &L, const VecDev *v, const Chunk *ch, int nch );          // (Jacobi) or before the first V-cycle (multigrid)
 void launch_mx_init1( const Launch &L, const VecDev *v, const Chunk *ch, int nch );         // (multigrid) after the first V-cycle
 void launch_mx_iter( const Launch &L, const VecDev *v, const Chunk *ch, int nch );          // (Jacobi) one iteration
 void launch_mx_spmv_update( const Launch &L, const VecDev *v, const Chunk *ch, int nch );   // (multigrid) before the V-cycle
 void launch_mx_rz_p( const Launch &L, const VecDev *v, const Chunk *ch, int nch );          // (multigrid) after the V-cycle
+// pcg.cu: the blocks of a launch for problems of these row counts (at most PCG_MAX_BLOCKS of them), { problem, rank, team
+// size, team } each; returns the cluster size of the launch, 0 for a cooperative one
+int pcg_teams( const std::vector<int> &rows, std::vector<int4> &teams );
+// up to `burst` iterations of every problem's CG, the start included when its SC_ITER is negative; bars: a counter a problem
+cudaError_t launch_pcg( const Launch &L, const PcgProb *probs, const int4 *teams, int nblocks, int cluster, int nteams, const MgLevel *chain,
+                        const VecDev *vs, int burst, unsigned *bars );
 // mg.cu
 void launch_mg_level0( const Launch &L, const MgLevel *lv, const VecDev *vs, const Chunk *ch, int nch );
 void launch_mg_coarsen( const Launch &L, const MgLevel *lv, int nprob, const Chunk *ch, int nch, ErrRec *err );

@@ -6,6 +6,7 @@
 // operator P^T A P of the piecewise-constant prolongation, which is again a graph Laplacian: off-diagonals
 // c_IJ = sum of the c_ij between the two aggregates, dia = the row sum.  The coarsest level (<= MG_BOTTOM rows)
 // is solved exactly by the dense inverse of A + mu 1 1^T, which acts as the pseudo-inverse on zero-sum vectors.
+// (The cycle's kernels here are the mixed CG's; the FP64 CG runs the same cycle inside its own launch, pcg.cu.)
 // One V(1,1)-cycle with damped Jacobi on both sides and an over-corrected coarse correction (symmetric, so it is a
 // valid CG preconditioner), all in FP32:
 // the outer CG stays in FP64 and plays the part of the iterative refinement.
@@ -294,14 +295,14 @@ __device__ __forceinline__ void mg_down_rows( const MgLevel &M, const VecDev *V,
         const int i0 = I * M.pack, i1 = in ? min( M.n, i0 + M.pack ) : i0;
         float acc = 0;
         for ( int i = i0 + sub; i < i1; i += MG_LANES ) {
-            float bi = top ? ( V->mixed ? V->r32[ i ] : float( V->r[ i ] ) ) : M.b[ i ];
+            float bi = top ? V->r32[ i ] : M.b[ i ];
             if ( top ) M.b[ i ] = bi;
             float xi = OMEGA * M.dinv[ i ] * bi;
             M.x[ i ] = xi;
             float ax = M.dia[ i ] * xi;
             for ( int e = M.rp[ i ]; e < M.rp[ i + 1 ]; ++e ) {
                 const int j = M.col[ e ];
-                float bj = top ? ( V->mixed ? V->r32[ j ] : float( V->r[ j ] ) ) : M.b[ j ];
+                float bj = top ? V->r32[ j ] : M.b[ j ];
                 ax -= M.val[ e ] * OMEGA * M.dinv[ j ] * bj;
             }
             acc += bi - ax;
@@ -311,8 +312,8 @@ __device__ __forceinline__ void mg_down_rows( const MgLevel &M, const VecDev *V,
     }
 }
 
-// prolongation of the next level's solution and post-smoothing for the fine rows [ i0, i1 ) of level M; level 0 writes z
-// (FP64, or z32 for the mixed CG); MG_LANES lanes per fine row
+// prolongation of the next level's solution and post-smoothing for the fine rows [ i0, i1 ) of level M; level 0 writes z32
+// (the mixed CG's); MG_LANES lanes per fine row
 __device__ __forceinline__ void mg_up_rows( const MgLevel &M, const VecDev &V, int i0, int i1, int t, int nt ) {
     const int sub = t % MG_LANES, per = nt / MG_LANES;
     const int end = i0 + ( ( i1 - i0 + per - 1 ) / per ) * per;
@@ -329,11 +330,8 @@ __device__ __forceinline__ void mg_up_rows( const MgLevel &M, const VecDev &V, i
             const float xi = M.x[ i ] + ALPHA * M.xn[ i / M.pack ];
             const float ai = M.dia[ i ] * xi - s;
             const float yi = xi + OMEGA * M.dinv[ i ] * ( M.b[ i ] - ai );
-            if ( M.level == 0 ) {
-                if ( V.mixed ) V.z32[ i ] = yi;
-                else V.z[ i ] = double( yi );
-            } else
-                M.y[ i ] = yi;
+            if ( M.level == 0 ) V.z32[ i ] = yi;
+            else M.y[ i ] = yi;
         }
     }
 }
