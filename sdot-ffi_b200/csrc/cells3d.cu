@@ -1,12 +1,10 @@
 // 3D Laguerre cells: ONE WARP PER CELL, the polyhedron in the warp's slice of shared memory.
 //
 // The cell is kept as its dual: every vertex is a triple of plane ids (a, b, c) -- the three faces meeting there,
-// ordered so that the triples form a consistently oriented triangulation of the sphere -- and its position is
-// ALWAYS re-solved from those three planes (solve3: FP64, seed frame), so no error accumulates along the
-// cuts (the reference re-solves its float vertices for the same reason, gpu/Cell3D.cuh:1093-1147).  A cut by the
-// plane P: lanes mark the vertices outside; for each directed edge (e0, e1) of a removed vertex whose twin (e1, e0)
-// belongs to a kept vertex, the new vertex (e0, e1, P) is created; kept vertices are compacted in order and the
-// new ones appended.  This is the dual-triangulation clipping published by Ray, Sokolov, Lefebvre and Levy
+// ordered so that the triples form a consistently oriented triangulation of the sphere -- and the clipped cell's positions
+// are re-solved from those three planes (solve3: FP64, seed frame).  A cut by the plane P: lanes mark the vertices outside;
+// for each directed edge (e0, e1) of a removed vertex whose twin (e1, e0) belongs to a kept vertex, the new vertex
+// (e0, e1, P) is created on that edge, in a removed vertex's place.  This is the dual-triangulation clipping published by Ray, Sokolov, Lefebvre and Levy
 // ("Meshless Voronoi on the GPU", ACM TOG 2018), written here for a warp.
 //
 // Candidates: the Morton grid, shell by shell around the seed's grid cell, 32 at a time, each candidate pre-tested
@@ -30,18 +28,17 @@ struct Cell3T {
     double vx[ VC ], vy[ VC ], vz[ VC ];
     double area[ 3 * VC ];                       // per (vertex, edge): the face-triangle contribution (integration)
     double nx[ PC ], ny[ PC ], nz[ PC ], no[ PC ];
-    int pid[ PC ];
+    int pid[ PC ], seq[ PC ];                    // seq: when the plane's candidate was met (the order of the facets)
     I va[ VC ], vb[ VC ], vc[ VC ];
     // the ADJACENCY: ad[ q ][ k ] is the vertex across edge q of vertex k (edge 0 = (va, vb), 1 = (vb, vc), 2 = (vc, va)),
     // the one holding the reversed directed edge; kept through every cut, so that no cut and no integration searches
     I ad[ 3 ][ VC ];
     unsigned char out[ VC ];
-    I nt[ VC ][ 3 ];                             // new triples of a cut; gaussians: the next entry of each face's list
-    I nk[ VC ];                                  // a cut: the kept vertex across each new vertex's first edge
-    I nidx[ VC ];                                // a cut: the index of each kept vertex after the compaction
+    I nt[ VC ][ 3 ];                             // a cut's new vertices: first two planes, removed end; gaussians: the next entry of each face's list
+    I nk[ VC ];                                  // a cut: the kept end of each new vertex's edge; then the holes
+    I nidx[ VC ];                                // a cut: the removed vertices; then where the vertices past the end move
     I e0t[ PC ], e1t[ PC ];                      // a cut: the new vertex whose first (second) plane is this one; NONE between cuts
-    double fmp[ PC ];                            // gaussians: the winding-angle part of each face's integral
-    double par[ PC ];                            // each face's integral (facets pass)
+    double par[ PC ];                            // gaussians: the winding-angle part of each face's integral; then the integral (facets pass)
     unsigned char used[ PC ];                    // plane compaction
     I remap[ PC ];
     double L;                                    // the farthest corner of the box from the seed (the tie band)
@@ -129,6 +126,7 @@ __device__ void init_box3( C3 &C, int lane, const double *lo, const double *hi, 
         C.nz[ lane ] = ax == 2 ? ( sg ? 1.0 : -1.0 ) : 0.0;
         C.no[ lane ] = sg ? hi[ ax ] - p : p - lo[ ax ];
         C.pid[ lane ] = -1 - lane;
+        C.seq[ lane ] = -1;
     }
     if ( lane < 8 ) {
         int sx = lane & 1, sy = ( lane >> 1 ) & 1, sz = ( lane >> 2 ) & 1;
@@ -167,7 +165,7 @@ __device__ bool compact_planes( C3 &C, int lane ) {
         for ( int p = 0; p < C.np; ++p ) {
             if ( ! used[ p ] ) continue;
             remap[ p ] = ( typename C3::I ) q;
-            C.nx[ q ] = C.nx[ p ]; C.ny[ q ] = C.ny[ p ]; C.nz[ q ] = C.nz[ p ]; C.no[ q ] = C.no[ p ]; C.pid[ q ] = C.pid[ p ];
+            C.nx[ q ] = C.nx[ p ]; C.ny[ q ] = C.ny[ p ]; C.nz[ q ] = C.nz[ p ]; C.no[ q ] = C.no[ p ]; C.pid[ q ] = C.pid[ p ]; C.seq[ q ] = C.seq[ p ];
             ++q;
         }
         C.np = q;
@@ -178,146 +176,169 @@ __device__ bool compact_planes( C3 &C, int lane ) {
     return C.np < PC;
 }
 
-// keep n . y <= off (a vertex within the tie band of the plane stays); false past a capacity
+// keep n . y <= off (a vertex within the tie band `tol` of the plane stays); false past a capacity.
+// A cut touches only what it changes: the removed vertices' slots take the new vertices (a cut that removes no face makes
+// two more than it removes), what is left of them is filled from the end, and the adjacency is rewritten at those vertices
+// alone -- the kept ones stay where they are.  A new vertex is taken ON the edge it cuts, between its kept end and its removed
+// one (one division); the clipped cell's vertices are re-solved from their three planes once, at the end (resolve3).
+// What bounds the clip: the instructions of a warp whose lanes hold 27 vertices and 5 new ones.  A cut that compacted every
+// vertex, remapped its adjacency and solved up to three new vertices a lane one after the other made most of a cell's; with
+// this one, the nearest of 32 candidates first, and the walk's tests and leaves filling the warp, a diagram takes, before ->
+// now: 1e5 weighted seeds 134 -> 66 ns a cell, 20,000 at a fit's weights 199 -> 101, 3,001 under gaussians 361 -> 266.
 template<class C3>
-__device__ bool wclip3( C3 &C, int lane, double nx, double ny, double nz, double off, int id ) {
+__device__ bool wclip3( C3 &C, int lane, double nx, double ny, double nz, double off, double tol, int id, int seq ) {
     const int nv = C.nv;
-    const double tol = tie_tol3( nx, ny, nz, off, C.L );
+    const unsigned below = ( 1u << lane ) - 1;
+    typedef typename C3::I I;
     int nout = 0;
     for ( int base = 0; base < nv; base += 32 ) {
         int k = base + lane;
         bool o = k < nv && nx * C.vx[ k ] + ny * C.vy[ k ] + nz * C.vz[ k ] - off > tol;
         if ( k < nv ) C.out[ k ] = o;
-        nout += __popc( __ballot_sync( FULL3, o ) );
+        const unsigned m = __ballot_sync( FULL3, o );
+        if ( o ) C.nidx[ nout + __popc( m & below ) ] = I( k );
+        nout += __popc( m );
     }
-    __syncwarp();
     if ( nout == 0 ) return true;
+    __syncwarp();
     if ( nout == nv ) {
         if ( lane == 0 ) C.nv = 0;
         __syncwarp();
         return true;
     }
     constexpr int VC = C3::VC, PC = C3::PC;
-    typedef typename C3::I I;
     const bool full = C.np >= PC;
-    __syncwarp();
-    if ( full && ! compact_planes( C, lane ) ) return false;
+    if ( full ) {
+        __syncwarp();
+        if ( ! compact_planes( C, lane ) ) return false;
+    }
     const int P = C.np;
     __syncwarp();
-    if ( lane == 0 ) { C.nx[ P ] = nx; C.ny[ P ] = ny; C.nz[ P ] = nz; C.no[ P ] = off; C.pid[ P ] = id; C.np = P + 1; }
-    __syncwarp();
-    // the boundary edges: directed edges of removed vertices whose twin (`ad`) is kept.  Each new vertex (e0, e1, P) is
-    // re-solved from its three planes; where that lands off the edge it replaces (three planes nearly through one
-    // line: a cut that grazes the edge), it is taken on the edge instead, from its kept end, where n . y = off.  Its
-    // position waits in `area` (free until the integration) while the kept vertices are compacted; the new vertex whose
-    // first (second) plane is p is recorded in e0t[ p ] (e1t[ p ]), which links the new vertices around the new face.
+    if ( lane == 0 ) { C.nx[ P ] = nx; C.ny[ P ] = ny; C.nz[ P ] = nz; C.no[ P ] = off; C.pid[ P ] = id; C.seq[ P ] = seq; C.np = P + 1; }
+    // the boundary edges: directed edges (e0, e1) of removed vertices whose twin (`ad`) is kept, one new vertex (e0, e1, P)
+    // each.  The new vertex whose first (second) plane is p is recorded in e0t[ p ] (e1t[ p ]), which links them around the
+    // new face
     int nnew = 0;
-    for ( int base = 0; base < nv; base += 32 ) {
-        int k = base + lane;
-        I tr[ 3 ][ 2 ];
-        int tt[ 3 ];
-        int cnt = 0;
-        if ( k < nv && C.out[ k ] ) {
-            int e[ 3 ] = { C.va[ k ], C.vb[ k ], C.vc[ k ] };
-            for ( int q = 0; q < 3; ++q ) {
-                const int t = C.ad[ q ][ k ];
-                if ( t != C3::NONE && ! C.out[ t ] ) { tr[ cnt ][ 0 ] = I( e[ q ] ); tr[ cnt ][ 1 ] = I( e[ ( q + 1 ) % 3 ] ); tt[ cnt ] = t; ++cnt; }
-            }
-        }
-        int inc = cnt;
+    for ( int base = 0; base < nout; base += 32 ) {
+        const bool in = base + lane < nout;
+        const int k = in ? C.nidx[ base + lane ] : 0;
+        int e[ 3 ] = { 0, 0, 0 }, t[ 3 ] = { 0, 0, 0 };
+        bool cut[ 3 ] = { false, false, false };
+        if ( in ) {
+            e[ 0 ] = C.va[ k ]; e[ 1 ] = C.vb[ k ]; e[ 2 ] = C.vc[ k ];
 #pragma unroll
-        for ( int o = 1; o < 32; o <<= 1 ) { int t = __shfl_up_sync( FULL3, inc, o ); if ( lane >= o ) inc += t; }
-        int total = __shfl_sync( FULL3, inc, 31 );
-        int at = nnew + inc - cnt;
-        for ( int q = 0; q < cnt; ++q ) {
-            const int j = at + q;
-            if ( j >= VC ) continue;
-            C.nt[ j ][ 0 ] = tr[ q ][ 0 ]; C.nt[ j ][ 1 ] = tr[ q ][ 1 ]; C.nt[ j ][ 2 ] = I( P );
-            const int t = tt[ q ];
-            C.nk[ j ] = I( t );
-            C.e0t[ tr[ q ][ 0 ] ] = I( j );
-            C.e1t[ tr[ q ][ 1 ] ] = I( j );
-            const double Rx = C.vx[ k ], Ry = C.vy[ k ], Rz = C.vz[ k ], Tx = C.vx[ t ], Ty = C.vy[ t ], Tz = C.vz[ t ];
-            double x, y, z;
-            solve3( C, tr[ q ][ 0 ], tr[ q ][ 1 ], P, x, y, z );
-            const double ex = Rx - Tx, ey = Ry - Ty, ez = Rz - Tz, e2 = ex * ex + ey * ey + ez * ez;
-            const double un = ( x - Tx ) * ex + ( y - Ty ) * ey + ( z - Tz ) * ez;     // u e2, u the edge parameter (NaN: no solve)
-            if ( ! ( un >= -1e-9 * e2 && un <= ( 1 + 1e-9 ) * e2 ) ) {
-                const double dT = nx * Tx + ny * Ty + nz * Tz - off, dR = nx * Rx + ny * Ry + nz * Rz - off;   // dR > tol >= dT
-                const double s = fmin( 1.0, fmax( 0.0, -dT / ( dR - dT ) ) );
-                x = Tx + s * ex; y = Ty + s * ey; z = Tz + s * ez;
+            for ( int q = 0; q < 3; ++q ) {
+                t[ q ] = C.ad[ q ][ k ];
+                cut[ q ] = t[ q ] != C3::NONE && ! C.out[ t[ q ] ];
             }
-            C.area[ j ] = x; C.area[ VC + j ] = y; C.area[ 2 * VC + j ] = z;
         }
-        nnew += total;
+#pragma unroll
+        for ( int q = 0; q < 3; ++q ) {
+            const unsigned m = __ballot_sync( FULL3, cut[ q ] );
+            const int j = nnew + __popc( m & below );
+            if ( cut[ q ] && j < VC ) {
+                const int e0 = e[ q ], e1 = e[ q == 2 ? 0 : q + 1 ];
+                C.nt[ j ][ 0 ] = I( e0 ); C.nt[ j ][ 1 ] = I( e1 ); C.nt[ j ][ 2 ] = I( k );
+                C.nk[ j ] = I( t[ q ] );
+                C.e0t[ e0 ] = I( j );
+                C.e1t[ e1 ] = I( j );
+            }
+            nnew += __popc( m );
+        }
     }
     __syncwarp();
     const int nkeep = nv - nout;
     const bool room = ! ( nkeep + nnew > VC || nnew >= VC );
-    // the new vertices make one cycle around the new face when every plane of the boundary is the first plane of exactly
-    // one new vertex and the second plane of exactly one; otherwise (a removed region that is not a disc, at the limits of
-    // rounding) the adjacency is searched again after the cut
-    bool cyc = true;
-    for ( int j = lane; j < nnew && room; j += 32 )
-        cyc = cyc && C.e0t[ C.nt[ j ][ 0 ] ] == j && C.e1t[ C.nt[ j ][ 1 ] ] == j && C.e0t[ C.nt[ j ][ 1 ] ] != C3::NONE &&
-              C.e1t[ C.nt[ j ][ 0 ] ] != C3::NONE;
-    cyc = __all_sync( FULL3, cyc );
     if ( ! room ) {
         for ( int j = lane; j < nnew && j < VC; j += 32 ) { C.e0t[ C.nt[ j ][ 0 ] ] = I( C3::NONE ); C.e1t[ C.nt[ j ][ 1 ] ] = I( C3::NONE ); }
         __syncwarp();
         return false;
     }
-    // compaction of the kept vertices, in order (destinations never pass their sources): first their new indices, then
-    // the moves, their adjacency mapped to those indices (an edge to a removed vertex gets its new vertex below)
-    int kept_before = 0;
-    for ( int base = 0; base < nv; base += 32 ) {
-        int k = base + lane;
-        bool keep = k < nv && ! C.out[ k ];
-        unsigned m = __ballot_sync( FULL3, keep );
-        if ( keep ) C.nidx[ k ] = I( kept_before + __popc( m & ( ( 1u << lane ) - 1 ) ) );
-        kept_before += __popc( m );
-    }
-    __syncwarp();
-    for ( int base = 0; base < nkeep + nout; base += 32 ) {
-        int k = base + lane;
-        bool keep = k < nv && ! C.out[ k ];
-        int dst = keep ? C.nidx[ k ] : 0;
-        double x = 0, y = 0, z = 0;
-        I a = 0, b = 0, c = 0, j0 = 0, j1 = 0, j2 = 0;
-        if ( keep ) {
-            x = C.vx[ k ]; y = C.vy[ k ]; z = C.vz[ k ]; a = C.va[ k ]; b = C.vb[ k ]; c = C.vc[ k ];
-            const int t0 = C.ad[ 0 ][ k ], t1 = C.ad[ 1 ][ k ], t2 = C.ad[ 2 ][ k ];
-            j0 = t0 == C3::NONE || C.out[ t0 ] ? I( C3::NONE ) : C.nidx[ t0 ];
-            j1 = t1 == C3::NONE || C.out[ t1 ] ? I( C3::NONE ) : C.nidx[ t1 ];
-            j2 = t2 == C3::NONE || C.out[ t2 ] ? I( C3::NONE ) : C.nidx[ t2 ];
-        }
-        __syncwarp();
-        if ( keep ) {
-            C.vx[ dst ] = x; C.vy[ dst ] = y; C.vz[ dst ] = z; C.va[ dst ] = a; C.vb[ dst ] = b; C.vc[ dst ] = c;
-            C.ad[ 0 ][ dst ] = j0; C.ad[ 1 ][ dst ] = j1; C.ad[ 2 ][ dst ] = j2;
-        }
-        __syncwarp();
-    }
-    // the new vertices, placed above: edge 0 (e0, e1) faces their kept vertex, edge 1 (e1, P) the new vertex that starts
-    // at e1, edge 2 (P, e0) the one that ends at e0; the kept vertex's edge (e1, e0) faces the new vertex
+    // the new vertices make one cycle around the new face when every plane of the boundary is the first plane of exactly
+    // one new vertex and the second plane of exactly one; otherwise (a removed region that is not a disc, at the limits of
+    // rounding) the adjacency is searched again after the cut.  Their positions wait in `area` (free until the integration):
+    // the removed ends are still read
+    bool cyc = true;
     for ( int j = lane; j < nnew; j += 32 ) {
-        const int d = nkeep + j, e0 = C.nt[ j ][ 0 ], e1 = C.nt[ j ][ 1 ];
+        const int e0 = C.nt[ j ][ 0 ], e1 = C.nt[ j ][ 1 ], k = C.nt[ j ][ 2 ], t = C.nk[ j ];
+        cyc = cyc && C.e0t[ e0 ] == j && C.e1t[ e1 ] == j && C.e0t[ e1 ] != C3::NONE && C.e1t[ e0 ] != C3::NONE;
+        const double Rx = C.vx[ k ], Ry = C.vy[ k ], Rz = C.vz[ k ], Tx = C.vx[ t ], Ty = C.vy[ t ], Tz = C.vz[ t ];
+        const double dT = nx * Tx + ny * Ty + nz * Tz - off, dR = nx * Rx + ny * Ry + nz * Rz - off;   // dR > tol >= dT
+        const double s = fmin( 1.0, fmax( 0.0, -dT / ( dR - dT ) ) );
+        C.area[ j ] = Tx + s * ( Rx - Tx ); C.area[ VC + j ] = Ty + s * ( Ry - Ty ); C.area[ 2 * VC + j ] = Tz + s * ( Rz - Tz );
+    }
+    cyc = __all_sync( FULL3, cyc );
+    __syncwarp();
+    // ... into the removed slots, then past the end: edge 0 (e0, e1) faces their kept vertex, edge 1 (e1, P) the new vertex
+    // that starts at e1, edge 2 (P, e0) the one that ends at e0; the kept vertex's edge (e1, e0) faces the new vertex
+    auto place = [&]( int j ) { return j < nout ? int( C.nidx[ j ] ) : nv + j - nout; };
+    for ( int j = lane; j < nnew; j += 32 ) {
+        const int d = place( j ), e0 = C.nt[ j ][ 0 ], e1 = C.nt[ j ][ 1 ], T = C.nk[ j ];
         C.va[ d ] = I( e0 ); C.vb[ d ] = I( e1 ); C.vc[ d ] = I( P );
         C.vx[ d ] = C.area[ j ]; C.vy[ d ] = C.area[ VC + j ]; C.vz[ d ] = C.area[ 2 * VC + j ];
-        const int T = C.nidx[ C.nk[ j ] ];
         C.ad[ 0 ][ d ] = I( T );
-        C.ad[ 1 ][ d ] = cyc ? I( nkeep + C.e0t[ e1 ] ) : I( C3::NONE );
-        C.ad[ 2 ][ d ] = cyc ? I( nkeep + C.e1t[ e0 ] ) : I( C3::NONE );
+        C.ad[ 1 ][ d ] = cyc ? I( place( C.e0t[ e1 ] ) ) : I( C3::NONE );
+        C.ad[ 2 ][ d ] = cyc ? I( place( C.e1t[ e0 ] ) ) : I( C3::NONE );
+        C.out[ d ] = 0;
         const int ta = C.va[ T ], tb = C.vb[ T ], tc = C.vc[ T ];
         const int qT = ( ta == e1 && tb == e0 ) ? 0 : ( ( tb == e1 && tc == e0 ) ? 1 : 2 );
         C.ad[ qT ][ T ] = I( d );
     }
     __syncwarp();
     for ( int j = lane; j < nnew; j += 32 ) { C.e0t[ C.nt[ j ][ 0 ] ] = I( C3::NONE ); C.e1t[ C.nt[ j ][ 1 ] ] = I( C3::NONE ); }
-    if ( lane == 0 ) C.nv = nkeep + nnew;
+    const int n1 = nkeep + nnew;
+    if ( nnew < nout ) {
+        // faces went with the cut: the slots left over, filled by the vertices past the new end, in order
+        int holes = 0;
+        for ( int base = 0; base < n1; base += 32 ) {
+            const int k = base + lane;
+            const bool h = k < n1 && C.out[ k ];
+            const unsigned m = __ballot_sync( FULL3, h );
+            if ( h ) C.nk[ holes + __popc( m & below ) ] = I( k );
+            holes += __popc( m );
+        }
+        __syncwarp();
+        int moved = 0;
+        for ( int base = n1; base < nv; base += 32 ) {
+            const int k = base + lane;
+            const bool mv = k < nv && ! C.out[ k ];
+            const unsigned m = __ballot_sync( FULL3, mv );
+            if ( mv ) {
+                const int h = C.nk[ moved + __popc( m & below ) ];
+                C.nidx[ k ] = I( h );
+                C.vx[ h ] = C.vx[ k ]; C.vy[ h ] = C.vy[ k ]; C.vz[ h ] = C.vz[ k ];
+                C.va[ h ] = C.va[ k ]; C.vb[ h ] = C.vb[ k ]; C.vc[ h ] = C.vc[ k ];
+                C.ad[ 0 ][ h ] = C.ad[ 0 ][ k ]; C.ad[ 1 ][ h ] = C.ad[ 1 ][ k ]; C.ad[ 2 ][ h ] = C.ad[ 2 ][ k ];
+            }
+            moved += __popc( m );
+        }
+        __syncwarp();
+        for ( int k = lane; k < n1; k += 32 )
+#pragma unroll
+            for ( int q = 0; q < 3; ++q ) {
+                const int t = C.ad[ q ][ k ];
+                if ( t != C3::NONE && t >= n1 ) C.ad[ q ][ k ] = C.nidx[ t ];
+            }
+    }
+    if ( lane == 0 ) C.nv = n1;
     __syncwarp();
     if ( ! cyc ) rebuild_adj( C, lane );
     return true;
+}
+
+// the clipped cell's vertices, each re-solved from its three planes, so that no error of the cuts stays in it (the reference
+// re-solves its float vertices for the same reason, gpu/Cell3D.cuh:1093-1147); a solve that lands away from the vertex (three
+// planes nearly through one line) is not taken
+template<class C3>
+__device__ __noinline__ void resolve3( C3 &C, int lane ) {
+    for ( int k = lane; k < C.nv; k += 32 ) {
+        double x, y, z;
+        solve3( C, C.va[ k ], C.vb[ k ], C.vc[ k ], x, y, z );
+        const double vx = C.vx[ k ], vy = C.vy[ k ], vz = C.vz[ k ];
+        const double d2 = ( x - vx ) * ( x - vx ) + ( y - vy ) * ( y - vy ) + ( z - vz ) * ( z - vz );
+        if ( d2 <= 1e-18 * ( vx * vx + vy * vy + vz * vz ) ) { C.vx[ k ] = x; C.vy[ k ] = y; C.vz[ k ] = z; }
+    }
+    __syncwarp();
 }
 
 // ---- the neighbour search ---------------------------------------------------------------------------------------------
@@ -348,9 +369,11 @@ __device__ __forceinline__ double radius2_3( const C3 &C, int lane ) {
 
 // the seeds of up to 32 grid cells (lane k: the range [ beg, beg + cnt ) of one cell) as candidates, 32 at a time:
 // each lane pre-tests one candidate against every vertex, then the cuts run in lane order
+// (of the 32, the one whose plane is nearest the seed cuts first: the far ones then often cut nothing; `met` counts the
+// candidates, so that the facets can be written in the order they were met)
 template<bool CNT, class C3>
 __device__ void cut_by_ranges3( C3 &C, const ProbDev &P, int lane, int s, double px, double py, double pz, double wi, int beg, int cnt,
-                                bool &overflow ) {
+                                int &met, bool &overflow ) {
     int inc = cnt;
 #pragma unroll
     for ( int o = 1; o < 32; o <<= 1 ) { int t = __shfl_up_sync( FULL3, inc, o ); if ( lane >= o ) inc += t; }
@@ -366,28 +389,38 @@ __device__ void cut_by_ranges3( C3 &C, const ProbDev &P, int lane, int s, double
         int j = obeg + ( t - oexc );
         bool valid = t < total && j != s;
         if constexpr ( CNT ) if ( P.gather ) count_reads( P, lane, G_CAND, __popc( __ballot_sync( FULL3, valid ) ) );
-        double qx = 0, qy = 0, qz = 0, off = 0;
+        double qx = 0, qy = 0, qz = 0, off = 0, tol = 1e300;
+        int key = 0x7fffffff;
         if ( valid ) {
             qx = P.pos[ 3 * ( size_t ) j ] - px;
             qy = P.pos[ 3 * ( size_t ) j + 1 ] - py;
             qz = P.pos[ 3 * ( size_t ) j + 2 ] - pz;
             double qw = P.w ? P.w[ j ] : 0.0;
-            off = 0.5 * ( ( wi - qw ) + ( qx * qx + qy * qy + qz * qz ) );
+            const double q2 = qx * qx + qy * qy + qz * qz;
+            off = 0.5 * ( ( wi - qw ) + q2 );
+            tol = tie_tol3( qx, qy, qz, off, C.L );
+            key = __float_as_int( float( off ) * rsqrtf( float( q2 ) ) );
+            key = key < 0 ? key ^ 0x7fffffff : key;
         }
         bool cuts = false;
-        const double tol = valid ? tie_tol3( qx, qy, qz, off, C.L ) : 0.0;
-        for ( int k = 0; k < C.nv && valid; ++k ) cuts |= qx * C.vx[ k ] + qy * C.vy[ k ] + qz * C.vz[ k ] - off > tol;
-        unsigned todo = __ballot_sync( FULL3, valid && cuts );
+        const int nv = C.nv;
+#pragma unroll 4
+        for ( int k = 0; k < nv; ++k ) cuts |= qx * C.vx[ k ] + qy * C.vy[ k ] + qz * C.vz[ k ] - off > tol;
+        unsigned todo = __ballot_sync( FULL3, cuts );
         while ( todo ) {
-            int k = __ffs( todo ) - 1;
-            todo &= todo - 1;
+            const bool mine = ( todo >> lane ) & 1;
+            const int least = __reduce_min_sync( FULL3, mine ? key : 0x7fffffff );
+            const unsigned at = __ballot_sync( FULL3, mine && key == least );
+            const int k = __ffs( at ? at : todo ) - 1;
+            todo &= ~( 1u << k );
             double nx = __shfl_sync( FULL3, qx, k ), ny = __shfl_sync( FULL3, qy, k ), nz = __shfl_sync( FULL3, qz, k );
-            double no = __shfl_sync( FULL3, off, k );
+            double no = __shfl_sync( FULL3, off, k ), nt = __shfl_sync( FULL3, tol, k );
             int nid = __shfl_sync( FULL3, j, k );
-            if ( ! wclip3( C, lane, nx, ny, nz, no, nid ) ) { overflow = true; break; }
+            if ( ! wclip3( C, lane, nx, ny, nz, no, nt, nid, met + t0 + k ) ) { overflow = true; break; }
             if ( C.nv == 0 ) break;
         }
     }
+    met += total;
 }
 
 constexpr int WALK_STACK3 = 96;      // at most 7 entries per level stay on the stack (12 levels)
@@ -401,8 +434,11 @@ constexpr int WALK_LEAF3 = 1;        // the walk's leaves: blocks of 2 x 2 x 2 g
 // vertices; only the claiming children are pushed
 template<bool CNT, class C3>
 __device__ void walk_pyramid3( C3 &C, const ProbDev &P, int lane, int s, double px, double py, double pz, double wi, const int *c0, int rd,
-                               int2 *stk, bool &overflow ) {
+                               int2 *stk, int &met, bool &overflow ) {
     const int *g = P.g;
+    // the leaves wait for one another, four of them to a warp (8 lanes each): one round of candidates tests what four would
+    // a quarter full each
+    int beg = 0, cnt = 0, leaves = 0;
     if ( lane == 0 ) stk[ 0 ] = make_int2( ( P.nlev - 1 ) << 22, 0 );
     int sp = 1;
     __syncwarp();
@@ -419,10 +455,10 @@ __device__ void walk_pyramid3( C3 &C, const ProbDev &P, int lane, int s, double 
         }
         if ( l <= WALK_LEAF3 ) {
             const int bw[ 3 ] = { a1[ 0 ] - a0[ 0 ] + 1, a1[ 1 ] - a0[ 1 ] + 1, a1[ 2 ] - a0[ 2 ] + 1 };   // at most 2 x 2 x 2
-            int beg = 0, cnt = 0;
+            const int in = lane & 7;
             bool tested = false, ranged = false;
-            if ( lane < bw[ 0 ] * bw[ 1 ] * bw[ 2 ] ) {
-                int x[ 3 ] = { a0[ 0 ] + lane % bw[ 0 ], a0[ 1 ] + ( lane / bw[ 0 ] ) % bw[ 1 ], a0[ 2 ] + lane / ( bw[ 0 ] * bw[ 1 ] ) };
+            if ( lane >> 3 == leaves && in < bw[ 0 ] * bw[ 1 ] * bw[ 2 ] ) {
+                int x[ 3 ] = { a0[ 0 ] + in % bw[ 0 ], a0[ 1 ] + ( in / bw[ 0 ] ) % bw[ 1 ], a0[ 2 ] + in / ( bw[ 0 ] * bw[ 1 ] ) };
                 bool walked = true;
                 for ( int a = 0; a < 3; ++a ) walked = walked && x[ a ] >= c0[ a ] - rd && x[ a ] <= c0[ a ] + rd;
                 const size_t gc = ( ( size_t ) x[ 2 ] * g[ 1 ] + x[ 1 ] ) * g[ 0 ] + x[ 0 ];
@@ -438,14 +474,17 @@ __device__ void walk_pyramid3( C3 &C, const ProbDev &P, int lane, int s, double 
                 count_reads( P, lane, G_GRID, __popc( __ballot_sync( FULL3, tested ) ) );
                 count_reads( P, lane, G_RANGE, __popc( __ballot_sync( FULL3, ranged ) ) );
             }
-            cut_by_ranges3<CNT>( C, P, lane, s, px, py, pz, wi, beg, cnt, overflow );
+            if ( ++leaves < 4 && sp > 0 ) continue;
+            cut_by_ranges3<CNT>( C, P, lane, s, px, py, pz, wi, beg, cnt, met, overflow );
             if ( overflow || C.nv == 0 ) return;
             R2 = radius2_3( C, lane );
+            beg = cnt = leaves = 0;
             continue;
         }
-        // the (up to 8) children, lane k the child k: in the grid, not all inside the walked shells, not empty
+        // the (up to 8) children, child `lane & 7` on four lanes: in the grid, not all inside the walked shells, not empty; does
+        // it claim a vertex of the cell?  (its four lanes share the vertices)
         int Y[ 3 ], b0[ 3 ], b1[ 3 ];
-        bool ok = lane < 8, inside = true;
+        bool ok = true, inside = true;
         for ( int a = 0; a < 3; ++a ) {
             Y[ a ] = 2 * X[ a ] + ( ( lane >> a ) & 1 );
             ok = ok && Y[ a ] < lev_dim( g[ a ], l - 1 );
@@ -454,33 +493,25 @@ __device__ void walk_pyramid3( C3 &C, const ProbDev &P, int lane, int s, double 
             inside = inside && b0[ a ] >= c0[ a ] - rd && b1[ a ] <= c0[ a ] + rd;
         }
         ok = ok && ! inside;
-        double cb = -1e300, ca[ 3 ] = { 0, 0, 0 }, lo[ 3 ] = { 0, 0, 0 }, hi[ 3 ] = { 0, 0, 0 }, dd = 0;
-        if constexpr ( CNT ) if ( P.gather ) count_reads( P, lane, G_NODE, __popc( __ballot_sync( FULL3, ok ) ) );
+        double dd = 0;
+        if constexpr ( CNT ) if ( P.gather ) count_reads( P, lane, G_NODE, __popc( __ballot_sync( FULL3, ok && lane < 8 ) ) );
+        bool may = false;
         if ( ok ) {
             const size_t rec = P.poff[ l - 1 ] + ( ( size_t ) Y[ 2 ] * lev_dim( g[ 1 ], l - 1 ) + Y[ 1 ] ) * lev_dim( g[ 0 ], l - 1 ) + Y[ 0 ];
-            cb = wmaj_b( P, rec );
+            const double cb = wmaj_b( P, rec );
             const double *am = P.wpyr + rec * 4;
-            ca[ 0 ] = am[ 0 ]; ca[ 1 ] = am[ 1 ]; ca[ 2 ] = am[ 2 ];
+            const double ca[ 3 ] = { am[ 0 ], am[ 1 ], am[ 2 ] };
+            double lo[ 3 ], hi[ 3 ];
             for ( int q = 0; q < 3; ++q ) { lo[ q ] = P.go[ q ] + b0[ q ] * P.gh[ q ]; hi[ q ] = P.go[ q ] + ( b1[ q ] + 1 ) * P.gh[ q ]; }
             dd = cells_dist2_3( P, b0, b1, px, py, pz );
-            ok = cb >= -1e299;
+            if ( cb >= -1e299 )
+                for ( int k = lane >> 3; k < C.nv && ! may; k += 4 ) {
+                    const double v[ 3 ] = { C.vx[ k ], C.vy[ k ], C.vz[ k ] }, Xp[ 3 ] = { px + v[ 0 ], py + v[ 1 ], pz + v[ 2 ] };
+                    may = wmaj_claims( ca, cb, lo, hi, Xp, v, 3, wi );
+                }
         }
-        // does each child claim a vertex of the cell?  (lanes over the vertices, the child's record broadcast)
-        unsigned todo = __ballot_sync( FULL3, ok ), claim = 0;
-        while ( todo ) {
-            const int c = __ffs( todo ) - 1;
-            todo &= todo - 1;
-            const double A[ 3 ] = { __shfl_sync( FULL3, ca[ 0 ], c ), __shfl_sync( FULL3, ca[ 1 ], c ), __shfl_sync( FULL3, ca[ 2 ], c ) };
-            const double B = __shfl_sync( FULL3, cb, c );
-            const double LO[ 3 ] = { __shfl_sync( FULL3, lo[ 0 ], c ), __shfl_sync( FULL3, lo[ 1 ], c ), __shfl_sync( FULL3, lo[ 2 ], c ) };
-            const double HI[ 3 ] = { __shfl_sync( FULL3, hi[ 0 ], c ), __shfl_sync( FULL3, hi[ 1 ], c ), __shfl_sync( FULL3, hi[ 2 ], c ) };
-            bool may = false;
-            for ( int k = lane; k < C.nv && ! may; k += 32 ) {
-                const double v[ 3 ] = { C.vx[ k ], C.vy[ k ], C.vz[ k ] }, Xp[ 3 ] = { px + v[ 0 ], py + v[ 1 ], pz + v[ 2 ] };
-                may = wmaj_claims( A, B, LO, HI, Xp, v, 3, wi );
-            }
-            if ( __any_sync( FULL3, may ) ) claim |= 1u << c;
-        }
+        unsigned claim = __ballot_sync( FULL3, may );
+        claim = ( claim | claim >> 8 | claim >> 16 | claim >> 24 ) & 0xff;
         // the claiming children pushed farthest first (equal distances in child order), so that the nearest is popped first
         int rank = 0;
 #pragma unroll
@@ -490,9 +521,13 @@ __device__ void walk_pyramid3( C3 &C, const ProbDev &P, int lane, int s, double 
         }
         const int nc = __popc( claim );
         if ( sp + nc > WALK_STACK3 ) return;               // cannot happen below 2^13 cells per side
-        if ( ( claim >> lane ) & 1 ) stk[ sp + rank ] = make_int2( ( ( l - 1 ) << 22 ) | ( Y[ 0 ] << 11 ) | Y[ 1 ], Y[ 2 ] );
+        if ( lane < 8 && ( ( claim >> lane ) & 1 ) ) stk[ sp + rank ] = make_int2( ( ( l - 1 ) << 22 ) | ( Y[ 0 ] << 11 ) | Y[ 1 ], Y[ 2 ] );
         sp += nc;
         __syncwarp();
+        if ( sp == 0 && leaves ) {                         // nothing left to expand: the waiting leaves
+            cut_by_ranges3<CNT>( C, P, lane, s, px, py, pz, wi, beg, cnt, met, overflow );
+            return;
+        }
     }
 }
 
@@ -603,14 +638,14 @@ __device__ __forceinline__ void edge_piece3( EdgeItem3 &I ) {
 }
 
 // the gaussian sums over the clipped cell: lane parts of the mass, of the first moment about the seed and of
-// int |y|^2 rho (seed frame); C.area receives each (vertex, edge) entry's part of its face integral and C.fmp each
+// int |y|^2 rho (seed frame); C.area receives each (vertex, edge) entry's part of its face integral and C.par each
 // face's winding-angle part (both summed over the gaussians, in gaussian order)
 template<class C3>
 __device__ __noinline__ void integrate_gauss3( C3 &C, const ProbDev &P, int lane, double px, double py, double pz, double &M, double &Fx,
                                                 double &Fy, double &Fz, double &S2 ) {
     const int nv = C.nv, np = C.np;
     for ( int k = lane; k < 3 * nv; k += 32 ) C.area[ k ] = 0;
-    for ( int p = lane; p < np; p += 32 ) C.fmp[ p ] = 0;
+    for ( int p = lane; p < np; p += 32 ) C.par[ p ] = 0;
     __syncwarp();
     if ( nv == 0 ) return;
     // each face's boundary entries (vertex k, edge q with e[ q ] the face), as a list in vertex order, built once for all
@@ -659,7 +694,7 @@ __device__ __noinline__ void integrate_gauss3( C3 &C, const ProbDev &P, int lane
         S2 += s2g * ( 3 * dM - h * b ) + 2 * ( cx * gx + cy * gy + cz * gz ) + ( cx * cx + cy * cy + cz * cz ) * dM;
     };
     // the face items are (gaussian of the group's selection, face), lane-consecutive; with at least 32 faces per
-    // gaussian, the 32 items of one round hold distinct faces, so their sums into `fmp` never meet, and each face's sum
+    // gaussian, the 32 items of one round hold distinct faces, so their sums into `par` never meet, and each face's sum
     // runs in gaussian order
     const int NE = 3 * nv, NPp = np > 32 ? np : 32;
     for ( int g0 = 0; g0 < ng; g0 += 32 ) {
@@ -771,7 +806,7 @@ __device__ __noinline__ void integrate_gauss3( C3 &C, const ProbDev &P, int lane
                 }
                 if ( Th != 0 ) {
                     const double I = KG * exp( -h * h * 0.5 / s2g ) * s2g * Th;
-                    C.fmp[ p ] += I;
+                    C.par[ p ] += I;
                     // the flux of the erfc field's constant part; at h = 0 its limit from the inner side
                     const double dM = h != 0 ? -h * INV4PI * mg * erfc( fabs( h ) * kr ) / fabs( h ) * Th : -INV4PI * mg * Th;
                     add( dM, I, h, nhx, nhy, nhz, cx, cy, cz, s2g );
@@ -827,6 +862,7 @@ __device__ __noinline__ bool clip3( C3 &C, const ProbDev &P, int prob, int s, in
     const double wi = P.w ? P.w[ s ] : 0.0;
     init_box3( C, lane, P.lo, P.hi, px, py, pz );
     bool overflow = false;
+    int met = 0;                 // candidates so far
     int c0[ 3 ];
     for ( int a = 0; a < 3; ++a ) {
         double x = a == 0 ? px : ( a == 1 ? py : pz );
@@ -861,7 +897,7 @@ __device__ __noinline__ bool clip3( C3 &C, const ProbDev &P, int prob, int s, in
                 count_reads( P, lane, G_GRID, __popc( __ballot_sync( FULL3, tested ) ) );
                 count_reads( P, lane, G_RANGE, __popc( __ballot_sync( FULL3, ranged ) ) );
             }
-            cut_by_ranges3<CNT>( C, P, lane, s, px, py, pz, wi, beg, cnt, overflow );
+            cut_by_ranges3<CNT>( C, P, lane, s, px, py, pz, wi, beg, cnt, met, overflow );
         }
         if ( C.nv == 0 || overflow ) break;
         double R2 = radius2_3( C, lane );
@@ -869,7 +905,8 @@ __device__ __noinline__ bool clip3( C3 &C, const ProbDev &P, int prob, int s, in
         if ( r * P.ghmin >= sqrt( R2 ) + sqrt( ex > 0 ? ex : 0.0 ) ) break;
         if ( P.wpyr && r >= SHELLS_FIRST && r < rmax && sqrt( R2 ) + sqrt( ex > 0 ? ex : 0.0 ) > ( r + 2 ) * P.ghmin ) { rd = r; break; }
     }
-    if ( rd >= 0 && C.nv > 0 && ! overflow ) walk_pyramid3<CNT>( C, P, lane, s, px, py, pz, wi, c0, rd, stk, overflow );
+    if ( rd >= 0 && C.nv > 0 && ! overflow ) walk_pyramid3<CNT>( C, P, lane, s, px, py, pz, wi, c0, rd, stk, met, overflow );
+    if ( ! overflow ) resolve3( C, lane );
     const int user = P.user[ s ];
     if ( overflow ) {
         // past the capacity of this warp's cell: the next pass rebuilds it -- but a trial diagram does not go past the big
@@ -967,7 +1004,7 @@ __device__ __noinline__ bool finish3( C3 &C, const ProbDev &P, int prob, int s, 
                     if ( C.vb[ k ] == p ) ar += C.area[ 3 * k + 1 ];
                     if ( C.vc[ k ] == p ) ar += C.area[ 3 * k + 2 ];
                 }
-                if ( gauss ) ar += C.fmp[ p ];
+                if ( gauss ) ar += C.par[ p ];
             }
             if ( p < C.np ) C.par[ p ] = seed_plane && ar > 0 ? ar : 0.0;
             nf += __popc( __ballot_sync( FULL3, seed_plane && ar > 0 ) );
@@ -989,14 +1026,15 @@ __device__ __noinline__ bool finish3( C3 &C, const ProbDev &P, int prob, int s, 
                 return true;
             }
         }
-        int written = 0;
         for ( int pbase = 0; pbase < C.np; pbase += 32 ) {
             int p = pbase + lane;
             const double ar = p < C.np ? C.par[ p ] : 0.0;
             const bool fac = ar > 0;
-            unsigned fm = __ballot_sync( FULL3, fac );
-            int slot = written + __popc( fm & ( ( 1u << lane ) - 1 ) );
             if ( fac ) {
+                // its place: the facets met before it
+                const int sq = C.seq[ p ];
+                int slot = 0;
+                for ( int q = 0; q < C.np; ++q ) slot += C.par[ q ] > 0 && C.seq[ q ] < sq;
                 double dist = sqrt( C.nx[ p ] * C.nx[ p ] + C.ny[ p ] * C.ny[ p ] + C.nz[ p ] * C.nz[ p ] );
                 int j = C.pid[ p ];
                 const int jid = user_order ? P.user[ j ] : j;
@@ -1008,7 +1046,6 @@ __device__ __noinline__ bool finish3( C3 &C, const ProbDev &P, int prob, int s, 
                     if ( P.nm ) P.nm[ at ] = rho * ar;
                 }
             }
-            written += __popc( fm );
         }
         if ( lane == 0 ) {
             P.nb[ row ] = nf;
@@ -1123,9 +1160,9 @@ __device__ bool cell3( C3 &C, const ProbDev &P, int prob, int s, int lane, unsig
 // once: the warps then mostly wait for instructions.  So the main kernel runs twice: pass 1 clips every gaussian cell and
 // stores it (its used planes and its vertices) in `Split3::mem`; pass 2 loads each one and integrates it.  A cell that
 // finds no room in `mem` is done whole by pass 2.  The record of a cell, 16-byte aligned: int nv, np (16 bytes), then
-// doubles vx, vy, vz [nv] and nx, ny, nz, no [np], ints pid [np], ushorts va, vb, vc [nv] and the adjacency ad [3][nv].
+// doubles vx, vy, vz [nv] and nx, ny, nz, no [np], ints pid, seq [np], ushorts va, vb, vc [nv] and the adjacency ad [3][nv].
 __device__ __forceinline__ size_t rec3_bytes( int nv, int np ) {
-    return ( 16 + size_t( 8 ) * ( 3 * nv + 4 * np ) + size_t( 4 ) * np + size_t( 12 ) * nv + 15 ) & ~size_t( 15 );
+    return ( 16 + size_t( 8 ) * ( 3 * nv + 4 * np ) + size_t( 8 ) * np + size_t( 12 ) * nv + 15 ) & ~size_t( 15 );
 }
 
 template<class C3>
@@ -1142,7 +1179,7 @@ __device__ long long store3( C3 &C, const Split3 &sp, int lane ) {
     if ( lane == 0 ) { reinterpret_cast<int *>( r )[ 0 ] = nv; reinterpret_cast<int *>( r )[ 1 ] = np; }
     double *v = reinterpret_cast<double *>( r + 16 ), *pl = v + 3 * nv;
     int *pid = reinterpret_cast<int *>( pl + 4 * np );
-    unsigned short *ids = reinterpret_cast<unsigned short *>( pid + np );
+    unsigned short *ids = reinterpret_cast<unsigned short *>( pid + 2 * np );
     for ( int k = lane; k < nv; k += 32 ) {
         v[ k ] = C.vx[ k ]; v[ nv + k ] = C.vy[ k ]; v[ 2 * nv + k ] = C.vz[ k ];
         ids[ k ] = C.va[ k ]; ids[ nv + k ] = C.vb[ k ]; ids[ 2 * nv + k ] = C.vc[ k ];
@@ -1153,6 +1190,7 @@ __device__ long long store3( C3 &C, const Split3 &sp, int lane ) {
     for ( int p = lane; p < np; p += 32 ) {
         pl[ p ] = C.nx[ p ]; pl[ np + p ] = C.ny[ p ]; pl[ 2 * np + p ] = C.nz[ p ]; pl[ 3 * np + p ] = C.no[ p ];
         pid[ p ] = C.pid[ p ];
+        pid[ np + p ] = C.seq[ p ];
     }
     return ( long long ) at;
 }
@@ -1163,7 +1201,7 @@ __device__ void load3( C3 &C, const Split3 &sp, long long at, int lane ) {
     const int nv = reinterpret_cast<const int *>( r )[ 0 ], np = reinterpret_cast<const int *>( r )[ 1 ];
     const double *v = reinterpret_cast<const double *>( r + 16 ), *pl = v + 3 * nv;
     const int *pid = reinterpret_cast<const int *>( pl + 4 * np );
-    const unsigned short *ids = reinterpret_cast<const unsigned short *>( pid + np );
+    const unsigned short *ids = reinterpret_cast<const unsigned short *>( pid + 2 * np );
     typedef typename C3::I I;
     for ( int k = lane; k < nv; k += 32 ) {
         C.vx[ k ] = v[ k ]; C.vy[ k ] = v[ nv + k ]; C.vz[ k ] = v[ 2 * nv + k ];
@@ -1176,6 +1214,7 @@ __device__ void load3( C3 &C, const Split3 &sp, long long at, int lane ) {
     for ( int p = lane; p < np; p += 32 ) {
         C.nx[ p ] = pl[ p ]; C.ny[ p ] = pl[ np + p ]; C.nz[ p ] = pl[ 2 * np + p ]; C.no[ p ] = pl[ 3 * np + p ];
         C.pid[ p ] = pid[ p ];
+        C.seq[ p ] = pid[ np + p ];
     }
     if ( lane == 0 ) { C.nv = nv; C.np = np; }
     __syncwarp();

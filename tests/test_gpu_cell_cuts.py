@@ -1,0 +1,49 @@
+"""Clips whose cuts take whole faces with them, and searches that go through the weights' pyramid, against the oracle
+(the same bars as test_gpu_cells.py)."""
+import numpy as np
+import pytest
+
+import sdot
+from test_gpu_cells import _compare, _pd
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("d", [2, 3])
+@pytest.mark.parametrize("layers", [1, 2, 5])
+def test_nested_shells(d, layers):
+    """a seed inside `layers` shells of 9 to 14 seeds, the outer ones met in any order: a nearer shell's cuts remove the faces
+    that the farther one's made, and the vertices left over are moved"""
+    rng = np.random.default_rng(10 * d + layers)
+    pos = [np.full((1, d), 0.5)]
+    for k in range(layers):
+        u = rng.normal(size=(14 - k, d))
+        pos.append(0.5 + (0.06 + 0.05 * k) * u / np.linalg.norm(u, axis=1)[:, None])
+    pos.append(rng.uniform(size=(40, d)))
+    pos = np.concatenate(pos)
+    _compare(pos[rng.permutation(len(pos))], None)
+
+
+@pytest.mark.parametrize("n", [33, 1000, 9001])
+@pytest.mark.parametrize("d", [2, 3])
+def test_steep_weights(d, n):
+    """weights half way to those of a map onto a fraction of the box, with noise: the global bound reaches far past the rings
+    and shells, so the pyramid is walked"""
+    rng = np.random.default_rng(n + d)
+    pos = rng.uniform(size=(n, d))
+    w = 0.5 * ((pos - 0.3) ** 2).sum(axis=1) + 0.05 * n ** (-2 / d) * rng.uniform(size=n)
+    _compare(pos, w)
+
+
+def test_facets_come_in_the_order_met():
+    """a row's neighbours come in the order the search meets them, whatever the order they cut in: by rings (2D: around the
+    polygon) and, in 3D, shells of grid cells"""
+    n = 4000
+    pos = np.random.default_rng(5).uniform(size=(n, 3))
+    nb, ids, _ = _pd(pos).hessian_rows()
+    g = np.ceil(1 / (2 / n) ** (1 / 3) * (1 - 1e-12)).astype(int)
+    lo, hi = np.minimum(pos.min(axis=0), 0), np.maximum(pos.max(axis=0), 1)
+    cell = np.clip(((pos - lo) / ((hi - lo) / g)).astype(int), 0, g - 1)
+    for i in range(0, n, 97):
+        shell = np.abs(cell[ids[i, : nb[i]]] - cell[i]).max(axis=1)
+        assert (np.diff(shell) >= 0).all(), (i, shell)
