@@ -864,9 +864,43 @@ __device__ __noinline__ void vjp2( const ProbDev &P, int lane, bool fac, int ui,
     }
 }
 
+// ---- the two passes of the gaussian cells -------------------------------------------------------------------------------
+// What bounds a whole cell: code.  The clip's walk and the quadrature with its error functions do not fit the instruction
+// cache together (13 of the 21 cycles between two instructions of a warp went into waiting for it), so the gaussian cells
+// of a diagram with facets are clipped and stored by one pass and integrated by the next: a diagram of 20,011 seeds under
+// 4 gaussians takes 61 ns a cell instead of 96.  Without facets there is no table to store in, and the cells stay whole.
+//
+// The polygon waits in the cell's own row of the neighbour table, which the second pass then writes, so the passes need no
+// memory of their own: its vertices in the coefficients (16 at most: a row holds CAP2 = 32 of them), its edges' ids in the
+// ids, its size in the count (-1: past 16 vertices, the second pass does the cell whole; -2: queued).  The lines are made
+// again from their seeds by the clip's own formula.  A caller's row shorter than that keeps its cells whole.
+constexpr int MROW2 = 16;
+__device__ __forceinline__ void store2( const WPoly &C, const ProbDev &P, size_t row, int lane ) {
+    if ( lane == 0 ) P.nb[ row ] = C.m <= MROW2 ? C.m : -1;
+    if ( C.m <= MROW2 && lane < C.m ) {
+        P.nc[ row * P.cap + 2 * lane ] = C.vx;
+        P.nc[ row * P.cap + 2 * lane + 1 ] = C.vy;
+        P.nid[ row * P.cap + lane ] = C.lid;
+    }
+}
+__device__ __forceinline__ void load2( WPoly &C, const ProbDev &P, size_t row, int m, int lane, double px, double py, double wi ) {
+    C.m = m;
+    C.vx = C.vy = C.lnx = C.lny = C.loff = 0;
+    C.lid = -1;
+    if ( lane < m ) {
+        C.vx = P.nc[ row * P.cap + 2 * lane ];
+        C.vy = P.nc[ row * P.cap + 2 * lane + 1 ];
+        C.lid = P.nid[ row * P.cap + lane ];
+        line64( P, C.lid, px, py, wi, C.lnx, C.lny, C.loff );
+    }
+    __syncwarp();                          // (read by every lane before the row is written)
+}
+
+// mode 0: every cell whole.  mode 1 (pass 1) and mode 2 (pass 2): the cells of a gaussian problem are clipped and stored by
+// pass 1 and integrated by pass 2 (the report too); the other problems are done whole by pass 1 and skipped by pass 2
 template<bool F32, bool CNT>
 __global__ void __launch_bounds__( 256, 3 ) k_cells2d( const ProbDev *__restrict__ probs, const Chunk *__restrict__ chunks, int nchunks,
-                                                    unsigned flags, ErrRec *err, OvfList *ovf ) {
+                                                    unsigned flags, ErrRec *err, OvfList *ovf, int mode ) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     __shared__ double sh_rep[ 8 ][ NB_REPORT ];
     __shared__ int2 sh_stk[ 8 ][ WALK_STACK ];
@@ -875,6 +909,9 @@ __global__ void __launch_bounds__( 256, 3 ) k_cells2d( const ProbDev *__restrict
         const Chunk ch = chunks[ c ];
         const ProbDev &P = probs[ ch.prob ];
         if ( ( P.fp32 != 0 ) != F32 ) continue;          // (block uniform: the other launch's)
+        const bool two = mode != 0 && P.dkind == D_GAUSS && facets && P.cap >= 2 * MROW2;
+        if ( mode == 2 && ! two ) continue;
+        const bool report = ( flags & F_REPORT ) && ! ( mode == 1 && two );
         double *rep = sh_rep[ warp ];          // this warp's report accumulators (lane 0 updates them)
         if ( lane == 0 ) {
             Rep r0;
@@ -886,17 +923,27 @@ __global__ void __launch_bounds__( 256, 3 ) k_cells2d( const ProbDev *__restrict
             const double px = P.pos[ 2 * ( size_t ) s ], py = P.pos[ 2 * ( size_t ) s + 1 ];
             const double wi = P.w ? P.w[ s ] : 0.0;
             WPoly C;
+            const int user = P.user[ s ];
+            const size_t trow = user_order ? user : s;
+            const int stored = two && mode == 2 ? P.nb[ trow ] : -1;
+            if ( stored == -2 ) {
+                // queued by pass 1.  Until the next pass its row of the table is empty (the limits kernel reads it before)
+                __syncwarp();
+                if ( lane == 0 ) P.nb[ trow ] = 0;
+                continue;
+            }
             bool overflow = false;
-            if constexpr ( F32 ) {
+            if ( stored >= 0 ) load2( C, P, trow, stored, lane, px, py, wi );
+            else if constexpr ( F32 ) {
                 WPolyF F;
                 clip2<CNT>( F, P, lane, s, px, py, wi, wmax, sh_stk[ warp ], overflow );
                 if ( ! overflow ) to_fp64( F, C, P, lane, px, py, wi );
             } else
                 clip2<CNT>( C, P, lane, s, px, py, wi, wmax, sh_stk[ warp ], overflow );
-            const int user = P.user[ s ];
             if ( overflow ) {
                 // past the 32 vertices a warp holds: the global-memory pass rebuilds it (report included)
                 if ( lane == 0 ) {
+                    if ( facets ) P.nb[ trow ] = two && mode == 1 ? -2 : 0;
                     if ( ovf ) {
                         int k = atomicAdd( &ovf->count, 1 );
                         if ( k < ovf->cap ) ovf->items[ k ] = OvfItem{ ch.prob, s };
@@ -904,6 +951,10 @@ __global__ void __launch_bounds__( 256, 3 ) k_cells2d( const ProbDev *__restrict
                     } else
                         record_error( P, err, 4, ch.prob, user, 33 );
                 }
+                continue;
+            }
+            if ( two && mode == 1 ) {
+                store2( C, P, trow, lane );
                 continue;
             }
             // ---- integration over the edges
@@ -929,6 +980,7 @@ __global__ void __launch_bounds__( 256, 3 ) k_cells2d( const ProbDev *__restrict
             int nf = __popc( fmask );
             if ( facets && nf > P.cap ) {
                 if ( lane == 0 ) {
+                    P.nb[ trow ] = 0;
                     if ( ovf ) {
                         int k = atomicAdd( &ovf->count, 1 );
                         if ( k < ovf->cap ) ovf->items[ k ] = OvfItem{ ch.prob, s };
@@ -969,7 +1021,7 @@ __global__ void __launch_bounds__( 256, 3 ) k_cells2d( const ProbDev *__restrict
                 }
             }
             if ( lane == 0 && P.mass ) P.mass[ user_order ? user : s ] = mass;
-            if ( ( flags & F_REPORT ) && lane == 0 ) {
+            if ( report && lane == 0 ) {
                 double nu = P.nu[ s ];
                 double e2 = fabs( nu - mass );
                 rep[ R_WORST ] = fmax( rep[ R_WORST ], e2 );
@@ -989,7 +1041,7 @@ __global__ void __launch_bounds__( 256, 3 ) k_cells2d( const ProbDev *__restrict
                 rep[ R_NEMPTY ] += mass > 0 ? 0.0 : 1.0;
             }
         }
-        if ( flags & F_REPORT ) finish_report( P, ch, sh_rep );
+        if ( report ) finish_report( P, ch, sh_rep );
     }
 }
 
@@ -1039,13 +1091,16 @@ void launch_cells2d( const Launch &L, const ProbDev *probs, const Chunk *chunks,
     // the counting instantiations only when the search's reads are counted (F_GATHER): the others compile without them
     const bool cnt = flags & F_GATHER;
     if ( clips & 1 ) {
-        if ( cnt ) k_cells2d<false, true><<<nchunks, 256, 0, L.stream>>>( probs, chunks, nchunks, flags, err, ovf );
-        else k_cells2d<false, false><<<nchunks, 256, 0, L.stream>>>( probs, chunks, nchunks, flags, err, ovf );
-        ++*L.launches;
+        auto *kern = cnt ? k_cells2d<false, true> : k_cells2d<false, false>;
+        const bool two = ( clips & 4 ) && ( flags & F_FACETS );
+        for ( int mode = two ? 1 : 0; mode <= ( two ? 2 : 0 ); ++mode ) {
+            kern<<<nchunks, 256, 0, L.stream>>>( probs, chunks, nchunks, flags, err, ovf, mode );
+            ++*L.launches;
+        }
     }
     if ( clips & 2 ) {
-        if ( cnt ) k_cells2d<true, true><<<nchunks, 256, 0, L.stream>>>( probs, chunks, nchunks, flags, err, ovf );
-        else k_cells2d<true, false><<<nchunks, 256, 0, L.stream>>>( probs, chunks, nchunks, flags, err, ovf );
+        auto *kern = cnt ? k_cells2d<true, true> : k_cells2d<true, false>;
+        kern<<<nchunks, 256, 0, L.stream>>>( probs, chunks, nchunks, flags, err, ovf, 0 );
         ++*L.launches;
     }
 }

@@ -454,7 +454,8 @@ void launch_trial( const Launch &L, const VecDev *v, const Chunk *ch, int nch );
 // cells2d.cu / cells3d.cu
 // the limits of the cells below the floor (one thread a cell; chunks of CHUNK cells over the LimDev array)
 void launch_limits2d( const Launch &L, const LimDev *lims, const Chunk *chunks, int nchunks );
-// clips: bit 0 the problems that clip in FP64, bit 1 those that clip in FP32 (ProbDev.fp32): one launch each
+// clips: bit 0 the problems that clip in FP64, bit 1 those that clip in FP32 (ProbDev.fp32): one launch each; bit 2: some of
+// the former are gaussian, whose diagrams with facets take two passes
 void launch_cells2d( const Launch &L, const ProbDev *probs, const Chunk *chunks, int nchunks, unsigned flags, ErrRec *err, OvfList *ovf,
                      int clips = 1 );
 // the queued big cells (count known on the host), polygons in `scratch` (VBIG vertices x 2 buffers per warp)

@@ -47,3 +47,22 @@ def test_facets_come_in_the_order_met():
     for i in range(0, n, 97):
         shell = np.abs(cell[ids[i, : nb[i]]] - cell[i]).max(axis=1)
         assert (np.diff(shell) >= 0).all(), (i, shell)
+
+
+@pytest.mark.parametrize("sides", [15, 16, 17, 31, 32, 33, 40])
+def test_gaussian_cells_in_two_passes(sides):
+    """under gaussians the cells of a diagram with facets are stored between two passes up to 16 vertices, done again past them,
+    queued past 32: their masses are the bits of the diagram without facets, and all is the oracle's"""
+    rng = np.random.default_rng(sides)
+    t = 2 * np.pi * (np.arange(sides) + 0.1 * rng.uniform(size=sides)) / sides
+    ring = 0.5 + 0.2 * np.stack([np.cos(t), np.sin(t)], axis=1)
+    far = rng.uniform(size=(300, 2))
+    far = far[np.linalg.norm(far - 0.5, axis=1) > 0.28]
+    pos = np.concatenate([far[:100], [[0.5, 0.5]], ring, far[100:]])
+    c, s = rng.uniform(0.2, 0.8, (3, 2)), rng.uniform(0.1, 0.3, 3)
+    g = sdot.SumOfGaussians(c, s, support_box=(np.zeros(2), np.ones(2)))
+    _compare(pos, None, (("gauss", c, s, g.normalized_version().weights), g))
+    args = (pos, np.zeros(len(pos)), np.zeros(2), np.ones(2), _pd(pos, dist=g)._density())
+    with_facets, whole = sdot._lib.cells(*args, want_facets=True), sdot._lib.cells(*args)
+    assert (with_facets["masses"] == whole["masses"]).all()
+    assert with_facets["nb_count"][min(100, len(far))] == sides
