@@ -22,7 +22,7 @@ namespace sdot {
 
 constexpr int MGT = 256;                // threads per block
 constexpr int MG_PAIRS = 1024;          // (column, value) pairs a warp gathers for one coarse row
-constexpr int MG_WARPS = 4;             // warps per block of the coarsening kernels
+constexpr int MG_WARPS = 16;            // warps per block of the coarsening kernels: a row each of a chunk's (MG_CCH)
 
 // ---- build -------------------------------------------------------------------------------------------------------------
 // level 0 from the FP64 CSR of the Newton Laplacian.  A coupling far above the rest of both its rows (two seeds 1e-12
@@ -69,24 +69,17 @@ __global__ void k_mg_level0( const MgLevel *__restrict__ lv, const VecDev *__res
 
 // the (column, value) pairs of coarse row I, gathered by one warp into shared memory as keys ( column << 11 | pair index )
 // and values by pair index, then sorted by key (a bitonic sort over the warp, padded to a power of 2): the pairs of
-// each coarse column form a run, in pair order.  Returns the pair count (-1: past MG_PAIRS)
+// each coarse column form a run, in pair order.  Returns the pair count (-1: past MG_PAIRS).  An aggregate's rows are
+// neighbours in the CSR, so its pairs are one stretch of it.  Bound by latency: a row at a time and 4 coarse rows a warp, a
+// level of 3,001 3D seeds took 110 us to count and 128 to fill, the hierarchy 583 us; so, with a warp a row, 240
 constexpr int MG_KEY_SHIFT = 11;                         // pair indices < 2048 (MG_PAIRS is 1024)
 __device__ int gather_sorted( const MgLevel &M, int I, long long *key, float *cv, int lane ) {
-    const int i0 = I * M.pack, i1 = min( M.n, i0 + M.pack );
-    int cnt = 0;
-    for ( int i = i0; i < i1; ++i ) {
-        const int b = M.rp[ i ], e = M.rp[ i + 1 ];
-        for ( int base = b; base < e; base += 32 ) {
-            const int k = base + lane, at = cnt + ( k - base );
-            if ( k < e && at < MG_PAIRS ) {
-                key[ at ] = ( ( long long ) ( M.col[ k ] / M.pack ) << MG_KEY_SHIFT ) | at;
-                cv[ at ] = M.val[ k ];
-            }
-            cnt += min( 32, e - base );
-        }
-    }
-    __syncwarp();
+    const int b = M.rp[ I * M.pack ], cnt = M.rp[ min( M.n, ( I + 1 ) * M.pack ) ] - b;
     if ( cnt > MG_PAIRS ) return -1;
+    for ( int k = lane; k < cnt; k += 32 ) {
+        key[ k ] = ( ( long long ) ( M.col[ b + k ] / M.pack ) << MG_KEY_SHIFT ) | k;
+        cv[ k ] = M.val[ b + k ];
+    }
     int n2 = 1;
     while ( n2 < cnt ) n2 <<= 1;
     for ( int k = cnt + lane; k < n2; k += 32 ) key[ k ] = 0x7fffffffffffffffll;
