@@ -395,35 +395,61 @@ __device__ void fit_slope( const double *mom, int dim, double *a ) {
     for ( int q = 0; q < dim; ++q ) if ( ! isfinite( a[ q ] ) ) { for ( int t = 0; t < dim; ++t ) a[ t ] = 0; return; }
 }
 
-// the levels above: moments summed from the children, the slope fitted, b reset (one block per problem, level by level)
-__global__ void __launch_bounds__( 1024 ) k_wpyr_up( const ProbDev *__restrict__ probs ) {
+// one node of level l: moments summed from the children, the slope fitted, b reset
+__device__ void wpyr_node( const ProbDev &P, int l, const int *d, const int *e, int X, int Y, int Z ) {
+    const int dim = P.dim, RS = dim + 1, MS = wmom_size( dim );
+    const long src = P.poff[ l - 1 ], at = P.poff[ l ] + ( long( Z ) * d[ 1 ] + Y ) * d[ 0 ] + X;
+    double mom[ 14 ];
+    for ( int k = 0; k < MS; ++k ) mom[ k ] = 0;
+    for ( int dz = 0; dz < ( dim == 3 ? 2 : 1 ); ++dz )
+        for ( int dy = 0; dy < 2; ++dy )
+            for ( int dx = 0; dx < 2; ++dx ) {
+                int x = 2 * X + dx, y = 2 * Y + dy, z = 2 * Z + dz;
+                if ( x < e[ 0 ] && y < e[ 1 ] && z < e[ 2 ] ) {
+                    const double *cm = P.wmom + ( src + ( long( z ) * e[ 1 ] + y ) * e[ 0 ] + x ) * MS;
+                    for ( int k = 0; k < MS; ++k ) mom[ k ] += cm[ k ];
+                }
+            }
+    for ( int k = 0; k < MS; ++k ) P.wmom[ at * MS + k ] = mom[ k ];
+    double a[ 3 ];
+    fit_slope( mom, dim, a );
+    for ( int q = 0; q < dim; ++q ) P.wpyr[ at * RS + q ] = a[ q ];
+    reinterpret_cast<unsigned long long *>( P.wpyr )[ at * RS + dim ] = dbl_order( -1e300 );
+}
+
+// the levels above the grid up to wtile( dim ): a block per tile, the tile being one node of that level with all its
+// descendants (64 nodes of level 1).  Bound by latency, a level's loads waiting for the level below: with one block per
+// problem for all the levels a diagram of 20,011 seeds waited 130 us for its index, one of 100,003 445 us; now 68 and 151
+__host__ __device__ constexpr int wtile( int dim ) { return dim == 2 ? 4 : 3; }
+__global__ void __launch_bounds__( 64 ) k_wpyr_tile( const ProbDev *__restrict__ probs ) {
+    const ProbDev &P = probs[ blockIdx.y ];
+    if ( ! P.wpyr ) return;
+    const int dim = P.dim, K = wtile( dim ), t = threadIdx.x;
+    int T[ 3 ] = { 1, 1, 1 };
+    for ( int a = 0; a < dim; ++a ) T[ a ] = lev_dim( P.g[ a ], K );
+    for ( int tile = blockIdx.x; tile < T[ 0 ] * T[ 1 ] * T[ 2 ]; tile += gridDim.x )
+        for ( int l = 1; l < P.nlev && l <= K; ++l ) {
+            int d[ 3 ] = { 1, 1, 1 }, e[ 3 ] = { 1, 1, 1 };
+            for ( int a = 0; a < dim; ++a ) { d[ a ] = lev_dim( P.g[ a ], l ); e[ a ] = lev_dim( P.g[ a ], l - 1 ); }
+            const int h = K - l, m = ( 1 << h ) - 1;
+            const int X = ( tile % T[ 0 ] << h ) + ( t & m ), Y = ( tile / T[ 0 ] % T[ 1 ] << h ) + ( t >> h & m );
+            const int Z = dim == 3 ? ( tile / ( T[ 0 ] * T[ 1 ] ) << h ) + ( t >> 2 * h ) : 0;
+            if ( t < 1 << dim * h && X < d[ 0 ] && Y < d[ 1 ] && Z < d[ 2 ] ) wpyr_node( P, l, d, e, X, Y, Z );
+            __syncthreads();
+        }
+}
+
+// the few nodes of the levels above the tiles: one block per problem, level by level
+__global__ void __launch_bounds__( 256 ) k_wpyr_up( const ProbDev *__restrict__ probs ) {
     const ProbDev &P = probs[ blockIdx.x ];
     if ( ! P.wpyr ) return;
-    const int dim = P.dim, RS = dim + 1, MS = wmom_size( dim );
-    for ( int l = 1; l < P.nlev; ++l ) {
+    const int dim = P.dim;
+    for ( int l = wtile( dim ) + 1; l < P.nlev; ++l ) {
         int d[ 3 ] = { 1, 1, 1 }, e[ 3 ] = { 1, 1, 1 };
         for ( int a = 0; a < dim; ++a ) { d[ a ] = lev_dim( P.g[ a ], l ); e[ a ] = lev_dim( P.g[ a ], l - 1 ); }
-        const long src = P.poff[ l - 1 ], dst = P.poff[ l ];
         const long cnt = long( d[ 0 ] ) * d[ 1 ] * d[ 2 ];
-        for ( long c = threadIdx.x; c < cnt; c += blockDim.x ) {
-            int X = int( c % d[ 0 ] ), Y = int( ( c / d[ 0 ] ) % d[ 1 ] ), Z = int( c / ( long( d[ 0 ] ) * d[ 1 ] ) );
-            double mom[ 14 ];
-            for ( int k = 0; k < MS; ++k ) mom[ k ] = 0;
-            for ( int dz = 0; dz < ( dim == 3 ? 2 : 1 ); ++dz )
-                for ( int dy = 0; dy < 2; ++dy )
-                    for ( int dx = 0; dx < 2; ++dx ) {
-                        int x = 2 * X + dx, y = 2 * Y + dy, z = 2 * Z + dz;
-                        if ( x < e[ 0 ] && y < e[ 1 ] && z < e[ 2 ] ) {
-                            const double *cm = P.wmom + ( src + ( long( z ) * e[ 1 ] + y ) * e[ 0 ] + x ) * MS;
-                            for ( int k = 0; k < MS; ++k ) mom[ k ] += cm[ k ];
-                        }
-                    }
-            for ( int k = 0; k < MS; ++k ) P.wmom[ ( dst + c ) * MS + k ] = mom[ k ];
-            double a[ 3 ];
-            fit_slope( mom, dim, a );
-            for ( int q = 0; q < dim; ++q ) P.wpyr[ ( dst + c ) * RS + q ] = a[ q ];
-            reinterpret_cast<unsigned long long *>( P.wpyr )[ ( dst + c ) * RS + dim ] = dbl_order( -1e300 );
-        }
+        for ( long c = threadIdx.x; c < cnt; c += blockDim.x )
+            wpyr_node( P, l, d, e, int( c % d[ 0 ] ), int( ( c / d[ 0 ] ) % d[ 1 ] ), int( c / ( long( d[ 0 ] ) * d[ 1 ] ) ) );
         __syncthreads();
     }
 }
@@ -475,9 +501,10 @@ __global__ void k_wpyr_b( const ProbDev *__restrict__ probs ) {
 void launch_wpyr( const Launch &L, const ProbDev *probs, int nprob ) {
     if ( nprob <= 0 ) return;
     k_wpyr0<<<dim3( 64, nprob ), 256, 0, L.stream>>>( probs );
-    k_wpyr_up<<<nprob, 1024, 0, L.stream>>>( probs );
+    k_wpyr_tile<<<dim3( 148, nprob ), 64, 0, L.stream>>>( probs );
+    k_wpyr_up<<<nprob, 256, 0, L.stream>>>( probs );
     k_wpyr_b<<<dim3( 64, nprob ), 256, 0, L.stream>>>( probs );
-    *L.launches += 3;
+    *L.launches += 4;
 }
 
 } // namespace sdot
