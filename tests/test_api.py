@@ -79,6 +79,32 @@ def test_exact_duplicates():
     assert len(exact_duplicates(np.random.default_rng(0).uniform(size=(100, 2)))[0]) == 0
 
 
+@pytest.mark.parametrize("case", ["few", "many", "grid", "zeros", "hash"])
+def test_exact_duplicates_are_those_of_a_search_over_whole_rows(case):
+    rng = np.random.default_rng(3)
+    p = rng.integers(0, 9, (500, 3)).astype(np.float32) if case == "many" else rng.uniform(size=(500, 2))
+    if case == "few":
+        p[[3, 77, 499]] = p[[400, 12, 0]]
+    if case == "grid":
+        p = np.stack(np.meshgrid(np.arange(20.), np.arange(25.)), axis=-1).reshape(-1, 2)
+    if case == "zeros":
+        p[:, 0] = rng.choice([0.0, -0.0], 500)
+        p[250:, 1] = p[:250, 1]
+    if case == "hash":                                     # rows of one hash and different values
+        def first(x):
+            h = np.atleast_1d(np.float64(x)).view(np.uint64) * np.uint64(0x9E3779B97F4A7C15)
+            return h ^ h >> np.uint64(29)
+        p[:250, 0], p[250:, 0] = 0.25, np.linspace(0.3, 0.9, 250)
+        p[250:, 1] = (p[:250, 1].copy().view(np.uint64) ^ first(0.25) ^ first(p[250:, 0])).view(np.float64)
+        p = p[np.isfinite(p).all(axis=1)]
+        p[0] = p[-1]
+    dup, rep = exact_duplicates(p)
+    first_at = {}
+    want = [first_at.setdefault(tuple(x + 0.0), i) for i, x in enumerate(np.asarray(p, float))]
+    assert list(dup) == [i for i, w in enumerate(want) if w != i]
+    assert list(rep) == [w for i, w in enumerate(want) if w != i]
+
+
 def test_public_names():
     for name in ("PowerDiagram", "Voronoi", "OtProblem", "Iterative", "Tuning", "OtNotConverged", "ot_solve", "SdotPlanNd", "SumOfDiracs",
                  "Image", "SumOfGaussians", "Box", "box_half_spaces", "KernelFailure"):
