@@ -17,7 +17,7 @@
 namespace sdot {
 
 constexpr int VT = 256;                       // threads per block of the vector kernels
-constexpr int VPT = VCHUNK / VT;              // rows per thread
+static_assert( VCHUNK <= VT, "the CSR kernels scan a chunk with a thread per row" );
 
 // deterministic block sum of NV values; thread 0 gets the result
 template<int NV>
@@ -88,17 +88,25 @@ __device__ __forceinline__ int find_in_row( const VecDev &V, int row, int key ) 
     return -1;
 }
 
+// a row by LAP_LANES lanes, a facet a lane: each walks its neighbour's row for its own.  Bound by the latency of those walks:
+// one thread a row walked them one after another (3,001 3D seeds: 38 us to count and 82 to fill, with the rest of the
+// assembly 29 us a launch; now 13)
+constexpr int LAP_LANES = 8;
 __global__ void __launch_bounds__( VT ) k_lap_count( const VecDev *__restrict__ vs, const Chunk *__restrict__ chunks, int nch ) {
     const Chunk ch = chunks[ blockIdx.x ];
     const VecDev &V = vs[ ch.prob ];
+    const int g = threadIdx.x % LAP_LANES;
     double tot = 0;
-    for ( int row = ch.begin + threadIdx.x; row < ch.end; row += VT ) {
+    for ( int base = ch.begin; base < ch.end; base += VT / LAP_LANES ) {
+        const int row = base + threadIdx.x / LAP_LANES;
         int cnt = 0;
-        const int nb = V.nb[ row ];
-        const int *ids = row_ids( V, row, nb );
-        for ( int k = 0; k < nb; ++k ) cnt += find_in_row( V, ids[ k ], row ) >= 0;
-        V.rowcnt[ row ] = cnt;
-        tot += cnt;
+        if ( row < ch.end ) {
+            const int nb = V.nb[ row ];
+            const int *ids = row_ids( V, row, nb );
+            for ( int k = g; k < nb; k += LAP_LANES ) cnt += find_in_row( V, ids[ k ], row ) >= 0;
+        }
+        for ( int o = LAP_LANES / 2; o > 0; o >>= 1 ) cnt += __shfl_xor_sync( 0xffffffffu, cnt, o );
+        if ( g == 0 && row < ch.end ) { V.rowcnt[ row ] = cnt; tot += cnt; }
     }
     double v[ 1 ] = { tot };
     block_sum<1>( v );
@@ -146,37 +154,38 @@ __global__ void __launch_bounds__( VT ) k_lap_fill( const VecDev *__restrict__ v
     const VecDev &V = vs[ ch.prob ];
     typedef cub::BlockScan<int, VT> Scan;
     __shared__ typename Scan::TempStorage tmp;
-    const int r0 = ch.begin + threadIdx.x * VPT;
-    int cnt[ VPT ], loc = 0;
-#pragma unroll
-    for ( int q = 0; q < VPT; ++q ) { int row = r0 + q; cnt[ q ] = row < ch.end ? V.rowcnt[ row ] : 0; loc += cnt[ q ]; }
+    __shared__ int off[ VT ];
+    const int mine = ch.begin + threadIdx.x;
     int ex;
-    Scan( tmp ).ExclusiveSum( loc, ex );
+    Scan( tmp ).ExclusiveSum( mine < ch.end ? V.rowcnt[ mine ] : 0, ex );
     if ( V.sc[ SC_NNZ ] > double( V.n ) * V.cap ) {                // past the CSR's capacity: empty rows (k_lap_scan)
-        for ( int q = 0; q < VPT && r0 + q < ch.end; ++q ) { V.row_ptr[ r0 + q ] = 0; V.dia[ r0 + q ] = 1.0; }
+        if ( mine < ch.end ) { V.row_ptr[ mine ] = 0; V.dia[ mine ] = 1.0; }
         return;
     }
-    int at = int( V.partials[ ( size_t ) ch.index * 4 + 1 ] ) + ex;
-#pragma unroll
-    for ( int q = 0; q < VPT; ++q ) {
-        int row = r0 + q;
-        if ( row >= ch.end ) break;
-        V.row_ptr[ row ] = at;
+    off[ threadIdx.x ] = int( V.partials[ ( size_t ) ch.index * 4 + 1 ] ) + ex;
+    __syncthreads();
+    const int lane = threadIdx.x & 31, g = lane % LAP_LANES, shift = lane - g;
+    const unsigned group = ( ( 1u << LAP_LANES ) - 1 ) << shift;
+    for ( int row = ch.begin + threadIdx.x / LAP_LANES; row < ch.end; row += VT / LAP_LANES ) {
+        int at = off[ row - ch.begin ];
         double s = 0;
         const int nb = V.nb[ row ];
         const int *ids = row_ids( V, row, nb );
         const double *cs = row_cs( V, row, nb );
-        for ( int k = 0; k < nb; ++k ) {
-            int j = ids[ k ];
-            int l = find_in_row( V, j, row );
-            if ( l < 0 ) continue;
-            double c = row < j ? cs[ k ] : row_cs( V, j, V.nb[ j ] )[ l ];
-            V.col[ at ] = j;
-            V.val[ at ] = c;
-            s += c;
-            ++at;
+        if ( g == 0 ) V.row_ptr[ row ] = at;
+        for ( int k0 = 0; k0 < nb; k0 += LAP_LANES ) {
+            const int k = k0 + g, j = k < nb ? ids[ k ] : 0, l = k < nb ? find_in_row( V, j, row ) : -1;
+            const double c = l < 0 ? 0.0 : row < j ? cs[ k ] : row_cs( V, j, V.nb[ j ] )[ l ];
+            const unsigned kept = __ballot_sync( group, l >= 0 ) >> shift;
+            if ( l >= 0 ) {
+                const int to = at + __popc( kept & ( ( 1u << g ) - 1 ) );
+                V.col[ to ] = j;
+                V.val[ to ] = c;
+            }
+            at += __popc( kept );
+            for ( int q = 0; q < LAP_LANES; ++q ) s += __shfl_sync( group, c, q, LAP_LANES );       // (in facet order)
         }
-        V.dia[ row ] = s > 0 ? s : 1.0;
+        if ( g == 0 ) V.dia[ row ] = s > 0 ? s : 1.0;
     }
 }
 
