@@ -872,8 +872,8 @@ __device__ __noinline__ void vjp2( const ProbDev &P, int lane, bool fac, int ui,
 //
 // The polygon waits in the cell's own row of the neighbour table, which the second pass then writes, so the passes need no
 // memory of their own: its vertices in the coefficients (16 at most: a row holds CAP2 = 32 of them), its edges' ids in the
-// ids, its size in the count (-1: past 16 vertices, the second pass does the cell whole; -2: queued).  The lines are made
-// again from their seeds by the clip's own formula.  A caller's row shorter than that keeps its cells whole.
+// ids, its size in the count (-1: past 16 vertices, the second pass does the cell whole; -2: queued); what the facets do not
+// overwrite of it is cleared.  The lines are made again from their seeds by the clip's own formula.  A caller's row shorter than that keeps its cells whole.
 constexpr int MROW2 = 16;
 __device__ __forceinline__ void store2( const WPoly &C, const ProbDev &P, size_t row, int lane ) {
     if ( lane == 0 ) P.nb[ row ] = C.m <= MROW2 ? C.m : -1;
@@ -1000,6 +1000,10 @@ __global__ void __launch_bounds__( 256, 3 ) k_cells2d( const ProbDev *__restrict
                     P.nid[ at ] = user_order ? P.user[ C.lid ] : C.lid;
                     P.nc[ at ] = cij;
                     if ( P.nm ) P.nm[ at ] = e.meas;
+                }
+                if ( lane >= nf ) {        // the polygon that waited here: past the facets the row reads as if it never had
+                    if ( lane < 2 * stored ) P.nc[ ( size_t ) row * P.cap + lane ] = 0;
+                    if ( lane < stored ) P.nid[ ( size_t ) row * P.cap + lane ] = -1;
                 }
                 if ( lane == 0 ) P.nb[ row ] = nf;
             }

@@ -66,3 +66,28 @@ def test_gaussian_cells_in_two_passes(sides):
     with_facets, whole = sdot._lib.cells(*args, want_facets=True), sdot._lib.cells(*args)
     assert (with_facets["masses"] == whole["masses"]).all()
     assert with_facets["nb_count"][min(100, len(far))] == sides
+
+
+@pytest.mark.parametrize("kind", ["uniform", "gauss", "image", "ring"])
+@pytest.mark.parametrize("d,n", [(2, 1), (2, 700), (2, 20011), (3, 700)])
+def test_the_rest_of_a_row_is_empty(d, n, kind):
+    """past its count a row of the neighbour tables reads (-1, 0, 0), whatever the cell waited in between two passes"""
+    if d == 3 and kind in ("image", "ring"):
+        pytest.skip("2D")
+    rng = np.random.default_rng(n + d)
+    pos, dist = rng.uniform(size=(n, d)), None
+    if kind in ("gauss", "ring"):
+        dist = sdot.SumOfGaussians(rng.uniform(0.2, 0.8, (3, d)), rng.uniform(0.1, 0.3, 3), support_box=(np.zeros(d), np.ones(d)))
+    if kind == "image":
+        dist = sdot.Image(rng.uniform(0.1, 1.0, size=(16, 16)), frame=[1 / 16, 1 / 16])
+    if kind == "ring" and n > 1:                           # a cell of 40 edges (queued) and its neighbours of few
+        t = 2 * np.pi * np.arange(40) / 40
+        pos[0], pos[1:41] = 0.5, 0.5 + 0.3 * np.stack([np.cos(t), np.sin(t)], axis=1)
+        pos = pos[:41]
+    nb, ids, coef, meas = _pd(pos, dist=dist).facets()
+    past = np.arange(ids.shape[1]) >= nb[:, None]
+    assert (ids[past] == -1).all() and (coef[past] == 0).all() and (meas[past] == 0).all()
+    assert (ids[~past] >= 0).all() and (coef[~past] > 0).all()
+    nb, ids, coef = _pd(pos, dist=dist).hessian_rows()
+    past = np.arange(ids.shape[1]) >= nb[:, None]
+    assert (ids[past] == -1).all() and (coef[past] == 0).all()
