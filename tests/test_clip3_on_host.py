@@ -1,0 +1,29 @@
+"""The device code of the 3D clip, run on the host by 32 lanes in step (warp_on_host.h), where what it holds between its cuts can
+be looked at: every vertex's links, whatever ties the seeds bring."""
+import os
+import subprocess
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+CSRC = os.path.join(HERE, "..", "sdot-ffi_b200", "csrc")
+
+
+@pytest.fixture(scope="module")
+def clip3(tmp_path_factory):
+    d = tmp_path_factory.mktemp("clip3")
+    src = open(os.path.join(CSRC, "cells3d.cu")).read()
+    (d / "clip3.inc").write_text(src[src.index("constexpr unsigned FULL3"):src.index("constexpr int WALK_STACK3")])
+    exe = str(d / "clip3")
+    # (an index past a fixed array ends the program)
+    subprocess.run(["g++", "-O1", "-std=c++17", "-fsanitize=bounds", "-fno-sanitize-recover", "-I", str(d), "-I", HERE, "-I", CSRC,
+                    "-I", "/usr/local/cuda/include", os.path.join(HERE, "clip3_on_host.cpp"), "-o", exe], check=True)
+    return lambda *args: [float(x) for x in subprocess.run([exe, *map(str, args)], check=True, capture_output=True, text=True).stdout.split()]
+
+
+def test_links_after_every_cut(clip3):
+    """seeds tied to the rounding of their coordinates, whose cuts now and then leave a boundary that is not one cycle: after every
+    cut each link of a cell is to a vertex of the cell that holds the reversed edge, or to none"""
+    cuts, wrong, searched = clip3("links", 2000)
+    assert cuts > 20000 and searched > 0
+    assert wrong == 0

@@ -91,3 +91,23 @@ def test_the_rest_of_a_row_is_empty(d, n, kind):
     nb, ids, coef = _pd(pos, dist=dist).hessian_rows()
     past = np.arange(ids.shape[1]) >= nb[:, None]
     assert (ids[past] == -1).all() and (coef[past] == 0).all()
+
+
+@pytest.mark.parametrize("jitter", [1e-15, 4e-15, 1e-14])
+@pytest.mark.parametrize("lattice", ["cubic", "face-centred"])
+def test_lattices_jittered_at_the_rounding(lattice, jitter):
+    """ties that rounding decides one by one.  A face moves by at most the jitter and the tie band (32 eps of lengths under 2), so a
+    cell of side h changes by 12 faces times (jitter + 3e-14) / h of its volume at most; the cells cover the box"""
+    m = 12
+    h = 1 / m
+    i = np.stack(np.meshgrid(*[np.arange(m)] * 3, indexing="ij"), axis=-1).reshape(-1, 3)
+    if lattice == "face-centred":
+        i = i[i.sum(axis=1) % 2 == 0]
+    rng = np.random.default_rng(len(i))
+    pos = (i + 0.5) * h + rng.uniform(-jitter, jitter, size=i.shape)
+    v = _pd(pos).measures
+    inner = ((i > 0) & (i < m - 1)).all(axis=1)
+    want = h ** 3 if lattice == "cubic" else 2 * h ** 3
+    bound = 12 * (jitter + 3e-14) / h
+    assert np.abs(v[inner] / want - 1).max() <= bound
+    assert abs(v.sum() - 1) <= bound
