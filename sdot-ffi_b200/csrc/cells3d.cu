@@ -43,7 +43,6 @@ struct Cell3T {
     I remap[ PC ];
     double L;                                    // the farthest corner of the box from the seed (the tie band)
     int nv, np;
-    int odd;                                     // 1 once a cut's boundary was not one cycle: `ad` may be one-sided
 };
 using Cell3 = Cell3T<128, 96, unsigned char>;            // the main kernel, in shared memory
 using Cell3B = Cell3T<1024, 256, unsigned short>;        // the big-cell pass: one warp a block, about 90 KB
@@ -102,15 +101,17 @@ __device__ __forceinline__ int twin_of( const C3 &C, int e0, int e1 ) {
     return -1;
 }
 
-// the adjacency of every vertex by search (the box, a loaded record, a cut whose boundary is not one cycle)
+// the adjacency of every vertex by search, after a cut whose boundary is not one cycle.  The links are MUTUAL, here as after
+// every other cut: where two vertices hold the same directed edge, its twin links to the first of them and the other's
+// own link is dropped.  A cut relies on it: the kept vertices with a link to a removed one are those that one links to
 template<class C3>
-__device__ void rebuild_adj( C3 &C, int lane ) {
+__device__ __noinline__ void rebuild_adj( C3 &C, int lane ) {
     typedef typename C3::I I;
     for ( int k = lane; k < C.nv; k += 32 ) {
         const int e[ 3 ] = { C.va[ k ], C.vb[ k ], C.vc[ k ] };
         for ( int q = 0; q < 3; ++q ) {
-            const int t = twin_of( C, e[ ( q + 1 ) % 3 ], e[ q ] );
-            C.ad[ q ][ k ] = t < 0 ? I( C3::NONE ) : I( t );
+            const int e0 = e[ q ], e1 = e[ q == 2 ? 0 : q + 1 ], t = twin_of( C, e1, e0 );
+            C.ad[ q ][ k ] = t < 0 || twin_of( C, e0, e1 ) != k ? I( C3::NONE ) : I( t );
         }
     }
     __syncwarp();
@@ -136,18 +137,20 @@ __device__ void init_box3( C3 &C, int lane, const double *lo, const double *hi, 
         int s = ( sx ? 1 : -1 ) * ( sy ? 1 : -1 ) * ( sz ? 1 : -1 );
         if ( s < 0 ) { int t = b; b = c; c = t; }
         C.va[ lane ] = a; C.vb[ lane ] = b; C.vc[ lane ] = c;
+        // across the edge of two planes, the corner on the other side of the third one's axis (searched, as after an odd cut, the
+        // corners' links took 4 of the 52 ns of a cell of 1e5 seeds)
+        C.ad[ 0 ][ lane ] = lane ^ ( 1 << ( c >> 1 ) ); C.ad[ 1 ][ lane ] = lane ^ 1; C.ad[ 2 ][ lane ] = lane ^ ( 1 << ( b >> 1 ) );
         C.vx[ lane ] = ( sx ? hi[ 0 ] : lo[ 0 ] ) - px;
         C.vy[ lane ] = ( sy ? hi[ 1 ] : lo[ 1 ] ) - py;
         C.vz[ lane ] = ( sz ? hi[ 2 ] : lo[ 2 ] ) - pz;
     }
     if ( lane == 0 ) {
-        C.nv = 8; C.np = 6; C.odd = 0;
+        C.nv = 8; C.np = 6;
         const double ex = fmax( hi[ 0 ] - px, px - lo[ 0 ] ), ey = fmax( hi[ 1 ] - py, py - lo[ 1 ] ), ez = fmax( hi[ 2 ] - pz, pz - lo[ 2 ] );
         C.L = sqrt( ex * ex + ey * ey + ez * ez );
     }
     for ( int p = lane; p < C3::PC; p += 32 ) { C.e0t[ p ] = typename C3::I( C3::NONE ); C.e1t[ p ] = typename C3::I( C3::NONE ); }
     __syncwarp();
-    rebuild_adj( C, lane );
 }
 
 // drops the planes no vertex uses (when the plane table is full); false if it cannot make room
@@ -180,9 +183,7 @@ __device__ bool compact_planes( C3 &C, int lane ) {
 // keep n . y <= off (a vertex within the tie band `tol` of the plane stays); false past a capacity.
 // A cut touches only what it changes: the removed vertices' slots take the new vertices (a cut that removes no face makes
 // two more than it removes), what is left of them is filled from the end, and the adjacency is rewritten at those vertices
-// alone -- the kept ones stay where they are.  That rests on the links being mutual: the kept vertices that link to a removed
-// one are then those it links to.  A search (rebuild_adj) may give one-sided links, where two vertices hold the same directed
-// edge, so a cell that needed one has its links searched after every later cut.  A new vertex is taken ON the edge it cuts, between its kept end and its removed
+// alone -- the kept ones stay where they are.  A new vertex is taken ON the edge it cuts, between its kept end and its removed
 // one (one division); the clipped cell's vertices are re-solved from their three planes once, at the end (resolve3).
 // What bounds the clip: the instructions of a warp whose lanes hold 27 vertices and 5 new ones.  A cut that compacted every
 // vertex, remapped its adjacency and solved up to three new vertices a lane one after the other made most of a cell's; with
@@ -259,9 +260,9 @@ __device__ bool wclip3( C3 &C, int lane, double nx, double ny, double nz, double
     }
     // the new vertices make one cycle around the new face when every plane of the boundary is the first plane of exactly
     // one new vertex and the second plane of exactly one; otherwise (a removed region that is not a disc, at the limits of
-    // rounding) the adjacency is searched again after the cut, and after the cell's later ones.  Their positions wait in `area`
-    // (free until the integration): the removed ends are still read
-    bool cyc = ! C.odd;
+    // rounding) the adjacency is searched again after the cut.  Their positions wait in `area` (free until the integration):
+    // the removed ends are still read
+    bool cyc = true;
     for ( int j = lane; j < nnew; j += 32 ) {
         const int e0 = C.nt[ j ][ 0 ], e1 = C.nt[ j ][ 1 ], k = C.nt[ j ][ 2 ], t = C.nk[ j ];
         cyc = cyc && C.e0t[ e0 ] == j && C.e1t[ e1 ] == j && C.e0t[ e1 ] != C3::NONE && C.e1t[ e0 ] != C3::NONE;
@@ -316,14 +317,14 @@ __device__ bool wclip3( C3 &C, int lane, double nx, double ny, double nz, double
             moved += __popc( m );
         }
         __syncwarp();
-        for ( int k = lane; cyc && k < n1; k += 32 )
+        for ( int k = lane; k < n1; k += 32 )
 #pragma unroll
             for ( int q = 0; q < 3; ++q ) {
                 const int t = C.ad[ q ][ k ];
                 if ( t != C3::NONE && t >= n1 ) C.ad[ q ][ k ] = C.nidx[ t ];
             }
     }
-    if ( lane == 0 ) { C.nv = n1; C.odd = ! cyc; }
+    if ( lane == 0 ) C.nv = n1;
     __syncwarp();
     if ( ! cyc ) rebuild_adj( C, lane );
     return true;

@@ -23,7 +23,7 @@ def clip3(tmp_path_factory):
 
 def test_links_after_every_cut(clip3):
     """seeds tied to the rounding of their coordinates, whose cuts now and then leave a boundary that is not one cycle: after every
-    cut each link of a cell is to a vertex of the cell that holds the reversed edge, or to none"""
-    cuts, wrong, searched = clip3("links", 2000)
-    assert cuts > 20000 and searched > 0
+    cut each link of a cell is to a vertex of the cell that holds the reversed edge and links back, or there is none"""
+    cuts, wrong, unlinked = clip3("links", 2000)
+    assert cuts > 20000 and unlinked > 0
     assert wrong == 0
