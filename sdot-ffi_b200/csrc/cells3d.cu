@@ -331,18 +331,43 @@ __device__ bool wclip3( C3 &C, int lane, double nx, double ny, double nz, double
 }
 
 // the clipped cell's vertices, each re-solved from its three planes, so that no error of the cuts stays in it (the reference
-// re-solves its float vertices for the same reason, gpu/Cell3D.cuh:1093-1147); a solve that lands away from the vertex (three
-// planes nearly through one line) is not taken
+// re-solves its float vertices for the same reason, gpu/Cell3D.cuh:1093-1147).  Mostly the solve lands within 1e-9 of the
+// vertex's length.  But a cut made while the cell was as large as the box leaves eps L in a vertex, more than that in a cell
+// of 1e-8 L: a solve from farther off is taken, too, if it lies on the three planes no worse than the vertex does and within
+// all the others by their tie bands (resolve_far3).  What is not taken leaves the cell: three planes nearly through one line
+template<class C3>
+__device__ __noinline__ void resolve_far3( C3 &C, int lane ) {
+    for ( int k = lane; k < C.nv; k += 32 ) {
+        const int own[ 3 ] = { C.va[ k ], C.vb[ k ], C.vc[ k ] };
+        const double vx = C.vx[ k ], vy = C.vy[ k ], vz = C.vz[ k ];
+        double x, y, z, now = 0, then = 0;       // the squared distances from the farthest of the three planes
+        solve3( C, own[ 0 ], own[ 1 ], own[ 2 ], x, y, z );
+        for ( int q = 0; q < 3; ++q ) {
+            const double nx = C.nx[ own[ q ] ], ny = C.ny[ own[ q ] ], nz = C.nz[ own[ q ] ], off = C.no[ own[ q ] ];
+            const double r = nx * x + ny * y + nz * z - off, s = nx * vx + ny * vy + nz * vz - off, n2 = nx * nx + ny * ny + nz * nz;
+            now = fmax( now, r * r / n2 );
+            then = fmax( then, s * s / n2 );
+        }
+        bool take = now <= then && fabs( x ) + fabs( y ) + fabs( z ) < 1e300;
+        for ( int p = 0; p < C.np && take; ++p )
+            take = C.nx[ p ] * x + C.ny[ p ] * y + C.nz[ p ] * z - C.no[ p ] <= tie_tol3( C.nx[ p ], C.ny[ p ], C.nz[ p ], C.no[ p ], C.L );
+        if ( take ) { C.vx[ k ] = x; C.vy[ k ] = y; C.vz[ k ] = z; }
+    }
+    __syncwarp();
+}
 template<class C3>
 __device__ __noinline__ void resolve3( C3 &C, int lane ) {
+    bool far = false;
     for ( int k = lane; k < C.nv; k += 32 ) {
         double x, y, z;
         solve3( C, C.va[ k ], C.vb[ k ], C.vc[ k ], x, y, z );
         const double vx = C.vx[ k ], vy = C.vy[ k ], vz = C.vz[ k ];
         const double d2 = ( x - vx ) * ( x - vx ) + ( y - vy ) * ( y - vy ) + ( z - vz ) * ( z - vz );
         if ( d2 <= 1e-18 * ( vx * vx + vy * vy + vz * vz ) ) { C.vx[ k ] = x; C.vy[ k ] = y; C.vz[ k ] = z; }
+        else far = true;
     }
     __syncwarp();
+    if ( __any_sync( FULL3, far ) ) resolve_far3( C, lane );
 }
 
 // ---- the neighbour search ---------------------------------------------------------------------------------------------
