@@ -576,7 +576,8 @@ int32_t sdot_linear_solve( sdot_context ctx, int64_t n, const int64_t *row_ptr, 
         // the team CG's launch: its problem (without a hierarchy), its blocks, its barrier
         const PcgProb one{ 0, 0, 0 };
         std::vector<int4> teams;
-        const int cluster = pcg_teams( std::vector<int>( 1, int( n ) ), teams );
+        std::vector<PcgLaunch> plan;
+        pcg_plan( std::vector<int>( 1, int( n ) ), pcg_blocks(), plan, teams );
         const size_t o2 = o1 + ( ( vch.size() * sizeof( Chunk ) + 255 ) & ~size_t( 255 ) ), o3 = o2 + 256;
         DevVec dd( c, o3 + teams.size() * sizeof( int4 ) );
         PcgProb *dprob = reinterpret_cast<PcgProb *>( ( char * ) dd.p + o2 );
@@ -621,7 +622,7 @@ int32_t sdot_linear_solve( sdot_context ctx, int64_t n, const int64_t *row_ptr, 
             for ( ;; ) {
                 if ( mixed )
                     for ( int s = 0; s < 32; ++s ) launch_mx_iter( L, dv, dch, int( vch.size() ) );
-                else CK( launch_pcg( L, dprob, dteams, int( teams.size() ), cluster, 1, nullptr, dv, 256, dbar ) );
+                else CK( launch_pcg( L, dprob, dteams, int( teams.size() ), plan[ 0 ].cluster, 1, nullptr, dv, 256, dbar ) );
                 CK( cudaMemcpyAsync( hsc, sc, sizeof( hsc ), cudaMemcpyDeviceToHost, c.stream ) );
                 CK( cudaStreamSynchronize( c.stream ) );
                 if ( hsc[ SC_CONV ] != 0 ) break;

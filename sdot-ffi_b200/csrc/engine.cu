@@ -1507,8 +1507,7 @@ struct VecBatch {
     std::vector<PcgProb> cprob;
     std::vector<MgLevel> cchain;
     std::vector<int> crows;
-    struct Group { int prob, nprob, block, nblock, cluster; };     // the launches: at most PCG_MAX_BLOCKS problems each
-    std::vector<Group> groups;
+    std::vector<PcgLaunch> groups;
     std::vector<int4> cteams;
     PcgProb *dcprob = nullptr;
     int4 *dcteams = nullptr;
@@ -1607,15 +1606,7 @@ struct VecBatch {
         parts.push_back( { build0.data(), build0.size() * sizeof( Chunk ) } );
         parts.push_back( { cprob.data(), cprob.size() * sizeof( PcgProb ) } );
         parts.push_back( { cchain.data(), cchain.size() * sizeof( MgLevel ) } );
-        groups.clear();
-        cteams.clear();
-        for ( int b = 0; b < int( crows.size() ); b += PCG_MAX_BLOCKS ) {
-            const int e = std::min( int( crows.size() ), b + PCG_MAX_BLOCKS );
-            std::vector<int4> t;
-            const int cl = pcg_teams( std::vector<int>( crows.begin() + b, crows.begin() + e ), t );
-            groups.push_back( Group{ b, e - b, int( cteams.size() ), int( t.size() ), cl } );
-            cteams.insert( cteams.end(), t.begin(), t.end() );
-        }
+        if ( ! crows.empty() ) pcg_plan( crows, pcg_blocks(), groups, cteams );
         const std::vector<unsigned> bars( crows.size(), 0u );
         parts.push_back( { cteams.data(), cteams.size() * sizeof( int4 ) } );
         parts.push_back( { bars.data(), bars.size() * sizeof( unsigned ) } );
@@ -1654,7 +1645,7 @@ struct VecBatch {
     }
     // up to `burst` iterations of a batch of the team CG
     void pcg( const Launch &L, int burst ) {
-        for ( const Group &g : groups )
+        for ( const PcgLaunch &g : groups )
             CK( launch_pcg( L, dcprob + g.prob, dcteams + g.block, g.nblock, g.cluster, g.nprob, dcchain, dv, burst, dcbars + g.prob ) );
     }
     // z = M^-1 r for every job

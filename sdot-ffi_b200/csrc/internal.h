@@ -433,9 +433,13 @@ void launch_mx_init1( const Launch &L, const VecDev *v, const Chunk *ch, int nch
 void launch_mx_iter( const Launch &L, const VecDev *v, const Chunk *ch, int nch );          // (Jacobi) one iteration
 void launch_mx_spmv_update( const Launch &L, const VecDev *v, const Chunk *ch, int nch );   // (multigrid) before the V-cycle
 void launch_mx_rz_p( const Launch &L, const VecDev *v, const Chunk *ch, int nch );          // (multigrid) after the V-cycle
-// pcg.cu: the blocks of a launch for problems of these row counts (at most PCG_MAX_BLOCKS of them), { problem, rank, team
-// size, team } each; returns the cluster size of the launch, 0 for a cooperative one
-int pcg_teams( const std::vector<int> &rows, std::vector<int4> &teams );
+// pcg.cu: the blocks that run together on the current device, PCG_MAX_BLOCKS at most
+int pcg_blocks();
+// the launches of the CG of problems of these row counts, of at most `most` blocks: the problems [ prob, prob + nprob ), the
+// blocks [ block, block + nblock ) of `teams`, { problem, rank, team size, team } each (counted from `prob`), the cluster size,
+// 0 for a cooperative launch
+struct PcgLaunch { int prob, nprob, block, nblock, cluster; };
+void pcg_plan( const std::vector<int> &rows, int most, std::vector<PcgLaunch> &launches, std::vector<int4> &teams );
 // up to `burst` iterations of every problem's CG, the start included when its SC_ITER is negative; bars: a counter a problem
 cudaError_t launch_pcg( const Launch &L, const PcgProb *probs, const int4 *teams, int nblocks, int cluster, int nteams, const MgLevel *chain,
                         const VecDev *vs, int burst, unsigned *bars );

@@ -24,6 +24,7 @@
 // the shares' sums in another; a block that plays several shares sums them one by one.  A solve is therefore bitwise the
 // same whatever its team's size -- which follows the batch's load -- and whatever else shares the launch.
 #include "internal.h"
+#include <algorithm>
 
 namespace sdot {
 
@@ -461,19 +462,17 @@ __global__ void __launch_bounds__( PCG_T, 1 ) k_pcg( const PcgProb *__restrict__
     else Pcg<4, 4>::run( V, chain + P.first, P.count, burst, small, T, sh, lv, Smem{ pcg_smem, pcg_smem + PCG_SMEM } );
 }
 
+// the blocks of a launch, at most: one an SM of the current device (a team's blocks run together)
 int pcg_blocks() {
-    static const int sms = [] {
-        int dev = 0, n = 0;
-        if ( cudaGetDevice( &dev ) != cudaSuccess || cudaDeviceGetAttribute( &n, cudaDevAttrMultiProcessorCount, dev ) != cudaSuccess ) n = 1;
-        return n < PCG_MAX_BLOCKS ? n : PCG_MAX_BLOCKS;
-    }();
-    return sms;
+    int dev = 0, n = 0;
+    if ( cudaGetDevice( &dev ) != cudaSuccess || cudaDeviceGetAttribute( &n, cudaDevAttrMultiProcessorCount, dev ) != cudaSuccess || n < 1 ) n = 1;
+    return n < PCG_MAX_BLOCKS ? n : PCG_MAX_BLOCKS;
 }
 
-// the blocks of each problem of a launch: one, the others in proportion to its rows, none more than it has shares.  When no
-// team passes 16 blocks every team is a cluster of one size
-int pcg_teams( const std::vector<int> &rows, std::vector<int4> &teams ) {
-    const int np = int( rows.size() ), most = pcg_blocks();
+// the blocks of each problem of a launch, of at most `most` (and as many problems): one, the others in proportion to its rows,
+// none more than it has shares.  When no team passes 16 blocks every team is a cluster of one size
+static int pcg_teams( const std::vector<int> &rows, int most, std::vector<int4> &teams ) {
+    const int np = int( rows.size() );
     std::vector<int> size( np, 1 );
     long sum = 0;
     int big = 0;
@@ -487,13 +486,24 @@ int pcg_teams( const std::vector<int> &rows, std::vector<int4> &teams ) {
     int cluster = 0;
     if ( big <= 16 ) {
         cluster = 1;
-        while ( cluster < big && 2 * cluster * np <= 128 ) cluster *= 2;
+        while ( cluster < big && 2 * cluster * np <= ( most < 128 ? most : 128 ) ) cluster *= 2;
         for ( int &s : size ) s = cluster;
     }
-    teams.clear();
     for ( int k = 0; k < np; ++k )
         for ( int q = 0; q < size[ k ]; ++q ) teams.push_back( make_int4( k, q, size[ k ], k ) );
     return cluster;
+}
+
+void pcg_plan( const std::vector<int> &rows, int most, std::vector<PcgLaunch> &launches, std::vector<int4> &teams ) {
+    launches.clear();
+    teams.clear();
+    const int np = int( rows.size() );
+    for ( int b = 0; b < np; b += most ) {
+        PcgLaunch l{ b, std::min( np, b + most ) - b, int( teams.size() ), 0, 0 };
+        l.cluster = pcg_teams( std::vector<int>( rows.begin() + b, rows.begin() + b + l.nprob ), most, teams );
+        l.nblock = int( teams.size() ) - l.block;
+        launches.push_back( l );
+    }
 }
 
 cudaError_t launch_pcg( const Launch &L, const PcgProb *probs, const int4 *teams, int nblocks, int cluster, int nteams, const MgLevel *chain,

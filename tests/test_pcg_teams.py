@@ -1,0 +1,82 @@
+"""How the team CG shares the GPU's blocks among the systems of a batch (host code of pcg.cu, built here by itself): every system
+gets a block, none more than it has shares, and no launch more than run together, on any number of SMs."""
+import os
+import subprocess
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+CSRC = os.path.join(HERE, "..", "sdot-ffi_b200", "csrc")
+MAIN = r"""
+#include <algorithm>
+#include <cstdio>
+#include <cstdlib>
+#include <iostream>
+#include "warp_on_host.h"
+#include "internal.h"
+namespace sdot {
+#include "teams.inc"
+}
+using namespace sdot;
+// SMs, the systems, their rows in; a line per launch: problems, cluster size, then { problem, rank, size, team } a block
+int main() {
+    int most, np;
+    std::cin >> most >> np;
+    std::vector<int> rows( np );
+    for ( int &n : rows ) std::cin >> n;
+    std::vector<PcgLaunch> launches;
+    std::vector<int4> t;
+    pcg_plan( rows, most, launches, t );
+    for ( const PcgLaunch &l : launches ) {
+        std::printf( "%d %d", l.nprob, l.cluster );
+        for ( int k = l.block; k < l.block + l.nblock; ++k ) std::printf( " %d %d %d %d", t[ k ].x, t[ k ].y, t[ k ].z, t[ k ].w );
+        std::printf( "\n" );
+    }
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def teams(tmp_path_factory):
+    d = tmp_path_factory.mktemp("teams")
+    src = open(os.path.join(CSRC, "pcg.cu")).read()
+
+    def piece(a, b):
+        i = src.index(a)
+        return src[i:src.index(b, i)]
+    (d / "teams.inc").write_text(piece("// rows of a share", "struct Team") + piece("// the blocks of each problem of a launch", "cudaError_t launch_pcg"))
+    (d / "main.cpp").write_text(MAIN)
+    exe = str(d / "teams")
+    subprocess.run(["g++", "-O1", "-std=c++17", "-I", str(d), "-I", HERE, "-I", CSRC, "-I", "/usr/local/cuda/include", str(d / "main.cpp"), "-o", exe], check=True)
+
+    def run(most, rows):
+        out = subprocess.run([exe], input=f"{most} {len(rows)} " + " ".join(map(str, rows)), check=True, capture_output=True, text=True).stdout
+        for line in out.splitlines():
+            nprob, cluster, *v = map(int, line.split())
+            yield nprob, cluster, list(zip(*[iter(v)] * 4))
+    return run
+
+
+def shares(n):
+    per = max(128, -(-(-(-n // 148)) // 32) * 32)
+    return -(-n // per)
+
+
+@pytest.mark.parametrize("sms", [148, 132, 20, 1])
+@pytest.mark.parametrize("rows", [[9], [1000], [1000000], [500] * 8, [100003] * 9, [100003] * 17, [20011] * 65, [2001] * 150, [1000000] + [100] * 147,
+                                  [1000000] + [3000] * 100, [4001, 100, 20011, 150]])
+def test_every_system_has_its_blocks(teams, sms, rows):
+    at = 0
+    for nprob, cluster, blocks in teams(sms, rows):
+        assert 1 <= nprob <= len(blocks) <= sms
+        of = {}
+        for problem, rank, size, team in blocks:
+            assert team == problem and 0 <= rank < size
+            of.setdefault(problem, []).append((rank, size))
+        assert sorted(of) == list(range(nprob))
+        for problem, team in of.items():
+            assert [r for r, _ in team] == list(range(len(team))) and all(size == len(team) for _, size in team)
+            # (a cluster's blocks past the shares do nothing)
+            assert cluster in (0, len(team)) and (cluster or len(team) <= shares(rows[at + problem]))
+        at += nprob
+    assert at == len(rows)
