@@ -577,7 +577,7 @@ int32_t sdot_linear_solve( sdot_context ctx, int64_t n, const int64_t *row_ptr, 
         const PcgProb one{ 0, 0, 0 };
         std::vector<int4> teams;
         std::vector<PcgLaunch> plan;
-        pcg_plan( std::vector<int>( 1, int( n ) ), pcg_blocks(), plan, teams );
+        pcg_plan( std::vector<int>( 1, int( n ) ), c.pcg_device(), plan, teams );
         const size_t o2 = o1 + ( ( vch.size() * sizeof( Chunk ) + 255 ) & ~size_t( 255 ) ), o3 = o2 + 256;
         DevVec dd( c, o3 + teams.size() * sizeof( int4 ) );
         PcgProb *dprob = reinterpret_cast<PcgProb *>( ( char * ) dd.p + o2 );

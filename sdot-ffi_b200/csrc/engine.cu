@@ -1606,7 +1606,7 @@ struct VecBatch {
         parts.push_back( { build0.data(), build0.size() * sizeof( Chunk ) } );
         parts.push_back( { cprob.data(), cprob.size() * sizeof( PcgProb ) } );
         parts.push_back( { cchain.data(), cchain.size() * sizeof( MgLevel ) } );
-        if ( ! crows.empty() ) pcg_plan( crows, pcg_blocks(), groups, cteams );
+        if ( ! crows.empty() ) pcg_plan( crows, c.pcg_device(), groups, cteams );
         const std::vector<unsigned> bars( crows.size(), 0u );
         parts.push_back( { cteams.data(), cteams.size() * sizeof( int4 ) } );
         parts.push_back( { bars.data(), bars.size() * sizeof( unsigned ) } );

@@ -63,6 +63,8 @@ struct Ctx {
     // the two passes of the gaussian 3D cells: their records and per-cell slots (grown on demand, see `split3_for`)
     Split3 split{};
     size_t split_slots = 0;
+    PcgDevice pcg{};                  // what its device runs at once of the team CG (asked for at the first CG, 5 us)
+    const PcgDevice &pcg_device() { if ( ! pcg.blocks ) pcg = sdot::pcg_device(); return pcg; }
     Timer timer;
     // the search's read counters of the standalone diagrams (sdot_cells) of dims 2 and 3, on request: [2][NB_GATHER][32]
     // on the device, and the cells those diagrams built

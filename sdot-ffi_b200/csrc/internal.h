@@ -433,13 +433,14 @@ void launch_mx_init1( const Launch &L, const VecDev *v, const Chunk *ch, int nch
 void launch_mx_iter( const Launch &L, const VecDev *v, const Chunk *ch, int nch );          // (Jacobi) one iteration
 void launch_mx_spmv_update( const Launch &L, const VecDev *v, const Chunk *ch, int nch );   // (multigrid) before the V-cycle
 void launch_mx_rz_p( const Launch &L, const VecDev *v, const Chunk *ch, int nch );          // (multigrid) after the V-cycle
-// pcg.cu: the blocks that run together on the current device, PCG_MAX_BLOCKS at most
-int pcg_blocks();
-// the launches of the CG of problems of these row counts, of at most `most` blocks: the problems [ prob, prob + nprob ), the
+// pcg.cu: what runs at once of the team CG on the current device: blocks (PCG_MAX_BLOCKS at most), clusters of 1, 2, 4, 8, 16
+struct PcgDevice { int blocks, clusters[ 5 ]; };
+PcgDevice pcg_device();
+// the launches of the CG of problems of these row counts: the problems [ prob, prob + nprob ), the
 // blocks [ block, block + nblock ) of `teams`, { problem, rank, team size, team } each (counted from `prob`), the cluster size,
 // 0 for a cooperative launch
 struct PcgLaunch { int prob, nprob, block, nblock, cluster; };
-void pcg_plan( const std::vector<int> &rows, int most, std::vector<PcgLaunch> &launches, std::vector<int4> &teams );
+void pcg_plan( const std::vector<int> &rows, const PcgDevice &D, std::vector<PcgLaunch> &launches, std::vector<int4> &teams );
 // up to `burst` iterations of every problem's CG, the start included when its SC_ITER is negative; bars: a counter a problem
 cudaError_t launch_pcg( const Launch &L, const PcgProb *probs, const int4 *teams, int nblocks, int cluster, int nteams, const MgLevel *chain,
                         const VecDev *vs, int burst, unsigned *bars );

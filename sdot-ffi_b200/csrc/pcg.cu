@@ -21,7 +21,8 @@
 // 5,000 rows: the vectors spread over a cluster's shared memories, whose network takes one address every two cycles.
 //
 // Sums: the rows are cut in SHARES by the row count alone, each summed by one block in a fixed tree, and every block folds
-// the shares' sums in another; a block that plays several shares sums them one by one.  A solve is therefore bitwise the
+// the shares' sums in another; a block that plays several shares sums each in the same tree (the trees of eight together, so
+// that it does not wait at the end of each: 148 systems of 20,011 rows, a block each, 576 -> 469 ms of CG).  A solve is therefore bitwise the
 // same whatever its team's size -- which follows the batch's load -- and whatever else shares the launch.
 #include "internal.h"
 #include <algorithm>
@@ -30,6 +31,7 @@ namespace sdot {
 
 constexpr int PCG_T = 768;                   // threads a block
 constexpr int PCG_W = PCG_T / 32;
+constexpr int PCG_SG = 8;                    // shares whose sums a block folds together
 constexpr int PCG_SMEM = 220 * 1024;         // dynamic shared memory of a block
 // the levels of at most this many rows are the first block's: a barrier and the steps' latency cost the team more than a
 // few rounds of the block's warps (1,251 rows: 6,000 cycles by one block, 8,000 with the team's two barriers)
@@ -82,18 +84,21 @@ SDOT_DEV double2 pcg_fold( const double2 *part, int ns, bool two ) {
     for ( int q = 0; q < ( PCG_MAX_BLOCKS + 31 ) / 32; ++q ) { a += v[ q ].x; b += v[ q ].y; }
     return make_double2( warp_sum( a ), warp_sum( b ) );
 }
-// the sums of one share over the block, written by thread 0 (a barrier of the team follows before they are read)
-SDOT_DEV void pcg_share( double a, double b, bool two, double2 *out, double2 *sh ) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+// the sums of the block's shares: a warp's part of each goes to `sh`, and after PCG_SG of them (or the last) the block folds
+// them together, a warp a share, and writes them to out[ share ] (a barrier of the team follows before they are read): a block
+// of many shares does not wait at the end of each
+SDOT_DEV void pcg_share( double a, double b, bool two, int s, int s0, int s1, double2 *out, double2 *sh ) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, at = ( s - s0 ) % PCG_SG;
     a = warp_sum( a );
     if ( two ) b = warp_sum( b );
-    if ( lane == 0 ) sh[ warp ] = make_double2( a, b );
+    if ( lane == 0 ) sh[ at * PCG_W + warp ] = make_double2( a, b );
+    if ( at + 1 < PCG_SG && s + 1 < s1 ) return;
     __syncthreads();
-    if ( warp == 0 ) {
-        const double2 v = lane < PCG_W ? sh[ lane ] : make_double2( 0, 0 );
+    if ( warp <= at ) {
+        const double2 v = lane < PCG_W ? sh[ warp * PCG_W + lane ] : make_double2( 0, 0 );
         a = warp_sum( v.x );
         if ( two ) b = warp_sum( v.y );
-        if ( lane == 0 ) *out = make_double2( a, b );
+        if ( lane == 0 ) out[ s - at + warp ] = make_double2( a, b );
     }
     __syncthreads();
 }
@@ -360,7 +365,7 @@ struct Pcg {
                             pq += p * q;
                         }
                     }
-                    pcg_share( pq, 0.0, false, part2 + par * ns + s, sh );
+                    pcg_share( pq, 0.0, false, s, s0, s1, part2 + par * ns, sh );
                 }
                 T.sync();
                 const double pq = pcg_fold( part2 + par * ns, ns, false ).x;
@@ -394,7 +399,7 @@ struct Pcg {
                         zz += ri * z;
                     }
                 }
-                pcg_share( rr, zz, L == 0, part2 + par * ns + s, sh );
+                pcg_share( rr, zz, L == 0, s, s0, s1, part2 + par * ns, sh );
             }
             T.sync();
             const double2 s = pcg_fold( part2 + par * ns, ns, L == 0 );
@@ -425,7 +430,7 @@ struct Pcg {
                             zz += r[ i ] * z;
                             pz[ i ] = make_double2( z, first ? 0.0 : p2[ i ] );
                         } );
-                    pcg_share( zz, 0.0, false, part2 + par * ns + s, sh );
+                    pcg_share( zz, 0.0, false, s, s0, s1, part2 + par * ns, sh );
                 }
                 T.sync();
                 rz1 = pcg_fold( part2 + par * ns, ns, false ).x;
@@ -445,7 +450,7 @@ struct Pcg {
 __global__ void __launch_bounds__( PCG_T, 1 ) k_pcg( const PcgProb *__restrict__ probs, const int4 *__restrict__ teams, const MgLevel *__restrict__ chain,
                                                  const VecDev *__restrict__ vs, int burst, unsigned *bars ) {
     extern __shared__ __align__( 16 ) char pcg_smem[];
-    __shared__ double2 sh[ PCG_W ];
+    __shared__ double2 sh[ PCG_SG * PCG_W ];
     __shared__ SLev lv[ MG_MAX_LEVELS ];
     __shared__ int dead;
     const int4 t = teams[ blockIdx.x ];
@@ -462,73 +467,109 @@ __global__ void __launch_bounds__( PCG_T, 1 ) k_pcg( const PcgProb *__restrict__
     else Pcg<4, 4>::run( V, chain + P.first, P.count, burst, small, T, sh, lv, Smem{ pcg_smem, pcg_smem + PCG_SMEM } );
 }
 
-// the blocks of a launch, at most: one an SM of the current device (a team's blocks run together)
-int pcg_blocks() {
-    int dev = 0, n = 0;
-    if ( cudaGetDevice( &dev ) != cudaSuccess || cudaDeviceGetAttribute( &n, cudaDevAttrMultiProcessorCount, dev ) != cudaSuccess || n < 1 ) n = 1;
-    return n < PCG_MAX_BLOCKS ? n : PCG_MAX_BLOCKS;
+// the launch of `blocks` blocks, in clusters of `cluster` (0: cooperative)
+static void pcg_config( cudaLaunchConfig_t &cfg, cudaLaunchAttribute &at, int blocks, int cluster ) {
+    cfg = {};
+    cfg.gridDim = dim3( blocks );
+    cfg.blockDim = dim3( PCG_T );
+    cfg.dynamicSmemBytes = PCG_SMEM;
+    cudaFuncSetAttribute( k_pcg, cudaFuncAttributeMaxDynamicSharedMemorySize, PCG_SMEM );      // (per device: set for every launch)
+    if ( cluster ) {
+        if ( cluster > 8 ) cudaFuncSetAttribute( k_pcg, cudaFuncAttributeNonPortableClusterSizeAllowed, 1 );
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = cluster; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
+    } else {
+        at.id = cudaLaunchAttributeCooperative;
+        at.val.cooperative = 1;
+    }
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
 }
 
-// the blocks of each problem of a launch, of at most `most` (and as many problems): one, the others in proportion to its rows,
-// none more than it has shares.  When no team passes 16 blocks every team is a cluster of one size
-static int pcg_teams( const std::vector<int> &rows, int most, std::vector<int4> &teams ) {
-    const int np = int( rows.size() );
-    std::vector<int> size( np, 1 );
+PcgDevice pcg_device() {
+    PcgDevice D{ 1, {} };
+    int dev = 0, n = 0;
+    if ( cudaGetDevice( &dev ) == cudaSuccess && cudaDeviceGetAttribute( &n, cudaDevAttrMultiProcessorCount, dev ) == cudaSuccess && n > 1 )
+        D.blocks = std::min( n, PCG_MAX_BLOCKS );
+    for ( int c = 0; c < 5; ++c ) {
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute at;
+        pcg_config( cfg, at, 1 << c, 1 << c );
+        if ( cudaOccupancyMaxActiveClusters( &D.clusters[ c ], k_pcg, &cfg ) != cudaSuccess ) { D.clusters[ c ] = 0; cudaGetLastError(); }
+    }
+    return D;
+}
+
+// the blocks of each of `np` problems of a launch of at most `D.blocks`: one, the others in proportion to its rows, none more than
+// it has shares.  When no team passes 16 blocks, every team is a cluster instead if they all run at once (of 148 SMs 15
+// clusters of 8 and 7 of 16) and a block's rows stay within PCG_CLUSTER_ROWS of that: a cluster's barriers are some 6 us an
+// iteration cheaper, a row more on a block costs 0.02 to 0.04.  Returns the cluster's size, 0 for none, and the ROUNDS of the
+// fullest block: a warp's turns over its shares
+constexpr int PCG_CLUSTER_ROWS = 200, PCG_ROUND = 8 * PCG_W;
+static int pcg_teams( const int *rows, int np, const PcgDevice &D, std::vector<int> &size, int &rounds ) {
+    size.assign( np, 1 );
     long sum = 0;
-    int big = 0;
-    for ( int n : rows ) sum += n;
+    int big = 0, load = 0, widest = 0;
+    for ( int k = 0; k < np; ++k ) { sum += rows[ k ]; widest = std::max( widest, rows[ k ] ); }
+    auto per = []( int a, int b ) { return ( a + b - 1 ) / b; };
+    auto shares = [&]( int k ) { return per( rows[ k ], pcg_share_rows( rows[ k ] ) ); };
     for ( int k = 0; k < np; ++k ) {
-        const int per = pcg_share_rows( rows[ k ] ), shares = ( rows[ k ] + per - 1 ) / per;
-        size[ k ] = 1 + int( double( most - np ) * rows[ k ] / double( sum ) );
-        if ( size[ k ] > shares ) size[ k ] = shares;
-        big = size[ k ] > big ? size[ k ] : big;
+        size[ k ] = std::min( shares( k ), 1 + int( double( D.blocks - np ) * rows[ k ] / double( sum ) ) );
+        big = std::max( big, size[ k ] );
+        load = std::max( load, per( rows[ k ], size[ k ] ) );
     }
     int cluster = 0;
-    if ( big <= 16 ) {
-        cluster = 1;
-        while ( cluster < big && 2 * cluster * np <= ( most < 128 ? most : 128 ) ) cluster *= 2;
-        for ( int &s : size ) s = cluster;
+    if ( big <= 16 && D.clusters[ 0 ] >= np ) {
+        int c = 0;
+        while ( ( 1 << c ) < big && D.clusters[ c + 1 ] >= np ) ++c;
+        if ( per( widest, 1 << c ) <= load + PCG_CLUSTER_ROWS ) { cluster = 1 << c; size.assign( np, cluster ); }
     }
-    for ( int k = 0; k < np; ++k )
-        for ( int q = 0; q < size[ k ]; ++q ) teams.push_back( make_int4( k, q, size[ k ], k ) );
+    rounds = 0;
+    for ( int k = 0; k < np; ++k ) rounds = std::max( rounds, per( shares( k ), size[ k ] ) * per( pcg_share_rows( rows[ k ] ), PCG_ROUND ) );
     return cluster;
 }
 
-void pcg_plan( const std::vector<int> &rows, int most, std::vector<PcgLaunch> &launches, std::vector<int4> &teams ) {
+// The launches of a batch.  A problem has a block at least, so with fewer problems a launch the SMs are shared out finer, but the
+// launches run one after the other.  Taken: the cut whose iteration takes least, a launch of R rounds taking 36 + 3.5 R + 0.1 R^2
+// us (its barriers and coarse levels; a round's latency; what no longer fits in shared memory).  Measured, ms of CG with so many
+// systems a launch: 65 of 20,011 rows, all 259, 33 199, 16 182, 8 219, 4 320; 17 of 100,003, all 279, 9 255, 4 212, 2 280, 1 435;
+// 33 of 50,003, all 264, 17 237, 8 183, 4 238
+void pcg_plan( const std::vector<int> &rows, const PcgDevice &D, std::vector<PcgLaunch> &launches, std::vector<int4> &teams ) {
+    const int np = int( rows.size() );
     launches.clear();
     teams.clear();
-    const int np = int( rows.size() );
-    for ( int b = 0; b < np; b += most ) {
-        PcgLaunch l{ b, std::min( np, b + most ) - b, int( teams.size() ), 0, 0 };
-        l.cluster = pcg_teams( std::vector<int>( rows.begin() + b, rows.begin() + b + l.nprob ), most, teams );
-        l.nblock = int( teams.size() ) - l.block;
-        launches.push_back( l );
+    std::vector<int> size;
+    long least = -1;
+    for ( int each = std::min( np, D.blocks ); each >= 1; each /= 2 ) {
+        std::vector<PcgLaunch> plan;
+        std::vector<int4> blocks;
+        long time = 0;
+        for ( int b = 0; b < np; b += each ) {
+            PcgLaunch l{ b, std::min( np, b + each ) - b, int( blocks.size() ), 0, 0 };
+            int R;
+            l.cluster = pcg_teams( rows.data() + b, l.nprob, D, size, R );
+            time += 360 + 35l * R + long( R ) * R;
+            for ( int k = 0; k < l.nprob; ++k )
+                for ( int q = 0; q < size[ k ]; ++q ) blocks.push_back( make_int4( k, q, size[ k ], k ) );
+            l.nblock = int( blocks.size() ) - l.block;
+            plan.push_back( l );
+        }
+        if ( least < 0 || time < least ) { least = time; launches = plan; teams = blocks; }
     }
 }
 
 cudaError_t launch_pcg( const Launch &L, const PcgProb *probs, const int4 *teams, int nblocks, int cluster, int nteams, const MgLevel *chain,
                         const VecDev *vs, int burst, unsigned *bars ) {
     if ( nblocks <= 0 ) return cudaSuccess;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3( nblocks );
-    cfg.blockDim = dim3( PCG_T );
-    cfg.dynamicSmemBytes = PCG_SMEM;
-    cfg.stream = L.stream;
-    cudaFuncSetAttribute( k_pcg, cudaFuncAttributeMaxDynamicSharedMemorySize, PCG_SMEM );      // (per device: set for every launch)
+    cudaLaunchConfig_t cfg;
     cudaLaunchAttribute at;
-    if ( cluster ) {
-        if ( cluster > 8 ) cudaFuncSetAttribute( k_pcg, cudaFuncAttributeNonPortableClusterSizeAllowed, 1 );
-        at.id = cudaLaunchAttributeClusterDimension;
-        at.val.clusterDim.x = cluster; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
-        bars = nullptr;
-    } else {
+    pcg_config( cfg, at, nblocks, cluster );
+    cfg.stream = L.stream;
+    if ( cluster ) bars = nullptr;
+    else {
         const cudaError_t e = cudaMemsetAsync( bars, 0, size_t( nteams ) * sizeof( unsigned ), L.stream );
         if ( e != cudaSuccess ) return e;
-        at.id = cudaLaunchAttributeCooperative;
-        at.val.cooperative = 1;
     }
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
     const cudaError_t e = cudaLaunchKernelEx( &cfg, k_pcg, probs, teams, chain, vs, burst, bars );
     ++*L.launches;
     return e;

@@ -7,6 +7,8 @@ import pytest
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "..", "sdot-ffi_b200", "csrc")
+#: the clusters of 1, 2, 4, 8 and 16 blocks that run at once (of 148 SMs: a B200's answer)
+CLUSTERS = {148: (148, 74, 33, 15, 7), 132: (132, 66, 30, 14, 6), 20: (20, 10, 4, 2, 1), 1: (1, 0, 0, 0, 0)}
 MAIN = r"""
 #include <algorithm>
 #include <cstdio>
@@ -18,15 +20,18 @@ namespace sdot {
 #include "teams.inc"
 }
 using namespace sdot;
-// SMs, the systems, their rows in; a line per launch: problems, cluster size, then { problem, rank, size, team } a block
+// SMs, the clusters of 1, 2, 4, 8 and 16 that run at once, the systems, their rows in; a line per launch: problems, cluster size, then { problem, rank, size, team } a block
 int main() {
-    int most, np;
-    std::cin >> most >> np;
+    PcgDevice D;
+    int np;
+    std::cin >> D.blocks;
+    for ( int &c : D.clusters ) std::cin >> c;
+    std::cin >> np;
     std::vector<int> rows( np );
     for ( int &n : rows ) std::cin >> n;
     std::vector<PcgLaunch> launches;
     std::vector<int4> t;
-    pcg_plan( rows, most, launches, t );
+    pcg_plan( rows, D, launches, t );
     for ( const PcgLaunch &l : launches ) {
         std::printf( "%d %d", l.nprob, l.cluster );
         for ( int k = l.block; k < l.block + l.nblock; ++k ) std::printf( " %d %d %d %d", t[ k ].x, t[ k ].y, t[ k ].z, t[ k ].w );
@@ -43,14 +48,16 @@ def teams(tmp_path_factory):
 
     def piece(a, b):
         i = src.index(a)
-        return src[i:src.index(b, i)]
-    (d / "teams.inc").write_text(piece("// rows of a share", "struct Team") + piece("// the blocks of each problem of a launch", "cudaError_t launch_pcg"))
+        return src[i:src.index(b, i)] + "\n"
+    (d / "teams.inc").write_text(piece("constexpr int PCG_T", "\n") + piece("constexpr int PCG_W", "\n") +
+                                 piece("// rows of a share", "struct Team") + piece("// the blocks of each of `np` problems", "cudaError_t launch_pcg"))
     (d / "main.cpp").write_text(MAIN)
     exe = str(d / "teams")
     subprocess.run(["g++", "-O1", "-std=c++17", "-I", str(d), "-I", HERE, "-I", CSRC, "-I", "/usr/local/cuda/include", str(d / "main.cpp"), "-o", exe], check=True)
 
-    def run(most, rows):
-        out = subprocess.run([exe], input=f"{most} {len(rows)} " + " ".join(map(str, rows)), check=True, capture_output=True, text=True).stdout
+    def run(sms, rows):
+        given = [sms, *CLUSTERS[sms], len(rows), *rows]
+        out = subprocess.run([exe], input=" ".join(map(str, given)), check=True, capture_output=True, text=True).stdout
         for line in out.splitlines():
             nprob, cluster, *v = map(int, line.split())
             yield nprob, cluster, list(zip(*[iter(v)] * 4))
@@ -69,6 +76,7 @@ def test_every_system_has_its_blocks(teams, sms, rows):
     at = 0
     for nprob, cluster, blocks in teams(sms, rows):
         assert 1 <= nprob <= len(blocks) <= sms
+        assert not cluster or nprob <= CLUSTERS[sms][cluster.bit_length() - 1]
         of = {}
         for problem, rank, size, team in blocks:
             assert team == problem and 0 <= rank < size
@@ -80,3 +88,14 @@ def test_every_system_has_its_blocks(teams, sms, rows):
             assert cluster in (0, len(team)) and (cluster or len(team) <= shares(rows[at + problem]))
         at += nprob
     assert at == len(rows)
+
+
+@pytest.mark.parametrize("rows", [[100003] * 8, [100003] * 9, [100003] * 17, [50003] * 33, [20011] * 65, [20011] * 80, [20011] * 148])
+def test_a_batch_of_large_systems_fills_the_sms(teams, rows):
+    """the rows of the fullest block of each launch, together, against the rows an SM has to do at least: a third more at most (the
+    clusters of one size left half of the SMs idle)"""
+    at = fullest = 0
+    for nprob, _, blocks in teams(148, rows):
+        fullest += max(-(-rows[at + problem] // size) for problem, _, size, _ in blocks)
+        at += nprob
+    assert fullest <= 4 / 3 * sum(rows) / 148
