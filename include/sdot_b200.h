@@ -138,6 +138,10 @@ int32_t sdot_context_set_counters(sdot_context ctx, int32_t on);
 /* the counts of `dim` (2 or 3) since the last reset: counts[5] = { cells built, candidate seeds, grid cells tested,
    grid ranges read, pyramid nodes }; synchronises the context's stream */
 int32_t sdot_context_gather_counters(sdot_context ctx, int32_t dim, uint64_t *counts, int32_t reset);
+/* how often a block of the CG asks at a barrier whether the others have come before it gives up (0: the default, some
+   seconds).  Blocks that the device does not run together would wait for good; a barrier that gives up ends the call with
+   SDOT_ERR_CUDA, and the context stays usable. */
+int32_t sdot_context_set_barrier_polls(sdot_context ctx, uint32_t polls);
 /* accumulated device time (ms), launches and units (seeds for the cells, rows x iterations for the CG) of a class
    since the last reset; synchronises the context's stream */
 int32_t sdot_context_kernel_stats(sdot_context ctx, int32_t kernel_class, double *ms, uint64_t *launches, double *units, int32_t reset);

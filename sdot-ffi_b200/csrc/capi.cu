@@ -177,6 +177,13 @@ int32_t sdot_context_set_counters( sdot_context ctx, int32_t on ) {
     return SDOT_OK;
 }
 
+int32_t sdot_context_set_barrier_polls( sdot_context ctx, uint32_t polls ) {
+    if ( ! ctx ) return SDOT_ERR_ARGS;
+    std::lock_guard<std::mutex> lock( ctx->mu );
+    ctx->c.pcg_polls = polls ? polls : PCG_POLLS;
+    return SDOT_OK;
+}
+
 int32_t sdot_context_gather_counters( sdot_context ctx, int32_t dim, uint64_t *counts, int32_t reset ) {
     if ( ! ctx || ! counts || ( dim != 2 && dim != 3 ) ) return SDOT_ERR_ARGS;
     std::lock_guard<std::mutex> lock( ctx->mu );
@@ -622,9 +629,11 @@ int32_t sdot_linear_solve( sdot_context ctx, int64_t n, const int64_t *row_ptr, 
             for ( ;; ) {
                 if ( mixed )
                     for ( int s = 0; s < 32; ++s ) launch_mx_iter( L, dv, dch, int( vch.size() ) );
-                else CK( launch_pcg( L, dprob, dteams, int( teams.size() ), plan[ 0 ].cluster, 1, nullptr, dv, 256, dbar ) );
+                else CK( launch_pcg( L, dprob, dteams, int( teams.size() ), plan[ 0 ].cluster, 1, nullptr, dv, 256, dbar, c.pcg_polls, c.derr ) );
                 CK( cudaMemcpyAsync( hsc, sc, sizeof( hsc ), cudaMemcpyDeviceToHost, c.stream ) );
+                CK( cudaMemcpyAsync( c.herr, c.derr, sizeof( ErrRec ), cudaMemcpyDeviceToHost, c.stream ) );
                 CK( cudaStreamSynchronize( c.stream ) );
+                check_errors( c, "sdot_linear_solve" );
                 if ( hsc[ SC_CONV ] != 0 ) break;
             }
             if ( iterations ) iterations[ k ] = hsc[ SC_FAIL ] != 0 ? -1 : int( hsc[ SC_ITER ] );

@@ -270,6 +270,7 @@ void check_errors( Ctx &c, const char *where ) {
                      e.needed );
     if ( e.code == SDOT_ERR_TOPOLOGY )
         throw Error( SDOT_ERR_TOPOLOGY, std::string( where ) + ": a cell's clip lost its topology (seed " + std::to_string( e.seed ) + ")", e.seed );
+    if ( e.code == SDOT_ERR_CUDA ) throw Error( SDOT_ERR_CUDA, "the CG: a barrier of its blocks waited in vain" );
     throw Error( e.code, std::string( where ) + ": device error", e.seed );
 }
 
@@ -1644,9 +1645,10 @@ struct VecBatch {
         launch_mg_bottom_build( L, dbottom, int( bottom.size() ) );
     }
     // up to `burst` iterations of a batch of the team CG
-    void pcg( const Launch &L, int burst ) {
+    void pcg( Ctx &c, int burst ) {
+        const Launch L = c.L();
         for ( const PcgLaunch &g : groups )
-            CK( launch_pcg( L, dcprob + g.prob, dcteams + g.block, g.nblock, g.cluster, g.nprob, dcchain, dv, burst, dcbars + g.prob ) );
+            CK( launch_pcg( L, dcprob + g.prob, dcteams + g.block, g.nblock, g.cluster, g.nprob, dcchain, dv, burst, dcbars + g.prob, c.pcg_polls, c.derr ) );
     }
     // z = M^-1 r for every job
     void vcycle( const Launch &L ) {
@@ -1730,7 +1732,7 @@ int mg_linear_solve( Ctx &c, const VecDev &V0, long nnz, double *hsc ) {
         }
     }
     for ( ;; ) {
-        if ( ! mixed ) B.pcg( L, PCG_BURST );
+        if ( ! mixed ) B.pcg( c, PCG_BURST );
         else for ( int k = 0; k < MG_BURST_SOLVE; ++k ) {
             if ( B.mg() ) {
                 launch_mx_spmv_update( L, B.dv, B.dch, nch );
@@ -2048,7 +2050,7 @@ void jobs_tick( Ctx &c, std::vector<SolveJob *> &jobs ) {
         for ( auto &v : cgc.v ) rows += v.n;
         c.timer.begin( c.stream, K_CG, rows );
         // the launch ends with the iteration that converges; in a batch it does not hold the others' diagrams up for long
-        cgc.pcg( L, jobs.size() == 1 ? PCG_BURST : ( with_diag.empty() ? PCG_BURST / 4 : PCG_BURST / 8 ) );
+        cgc.pcg( c, jobs.size() == 1 ? PCG_BURST : ( with_diag.empty() ? PCG_BURST / 4 : PCG_BURST / 8 ) );
         c.timer.end( c.stream, 1 );
     }
     for ( VecBatch *B : { &cgjx, &cgmx } ) {

@@ -64,6 +64,7 @@ struct Ctx {
     Split3 split{};
     size_t split_slots = 0;
     PcgDevice pcg{};                  // what its device runs at once of the team CG (asked for at the first CG, 5 us)
+    unsigned pcg_polls = PCG_POLLS;
     const PcgDevice &pcg_device() { if ( ! pcg.blocks ) pcg = sdot::pcg_device(); return pcg; }
     Timer timer;
     // the search's read counters of the standalone diagrams (sdot_cells) of dims 2 and 3, on request: [2][NB_GATHER][32]

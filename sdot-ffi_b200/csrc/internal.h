@@ -141,7 +141,7 @@ struct Chunk {
 
 // device-side error record (first error wins)
 struct ErrRec {
-    int code;      // 0 none, 4 capacity
+    int code;      // 0 none, 2 a barrier of the team CG gave up, 4 capacity, 7 topology (sdot_error)
     int kind;
     int prob;
     int seed;      // user index
@@ -221,6 +221,7 @@ struct MgLevel {
 struct PcgProb { int vec, first, count; };
 constexpr int PCG_SHARE = 128;         // rows one block of a CG team works on, at least (pcg.cu)
 constexpr int PCG_MAX_BLOCKS = 148;    // blocks of a launch, and problems
+constexpr unsigned PCG_POLLS = 1u << 21;     // polls of a team's barrier before it gives up (seconds)
 
 enum Scalar : int { SC_RZ = 0, SC_ALPHA, SC_BETA, SC_BNORM, SC_RNORM, SC_CONV, SC_ITER, SC_MEAN, SC_C, SC_TOL, SC_PQ, SC_FAIL, SC_NNZ,
                     SC_REFINE,      // mixed CG: 1 once the inner FP32 CG has converged (x += e, then the FP64 residual)
@@ -441,9 +442,10 @@ PcgDevice pcg_device();
 // 0 for a cooperative launch
 struct PcgLaunch { int prob, nprob, block, nblock, cluster; };
 void pcg_plan( const std::vector<int> &rows, const PcgDevice &D, std::vector<PcgLaunch> &launches, std::vector<int4> &teams );
-// up to `burst` iterations of every problem's CG, the start included when its SC_ITER is negative; bars: a counter a problem
+// up to `burst` iterations of every problem's CG, the start included when its SC_ITER is negative; bars: a counter a problem; a
+// barrier that gives up after `polls` fails its problem and is recorded in `err`
 cudaError_t launch_pcg( const Launch &L, const PcgProb *probs, const int4 *teams, int nblocks, int cluster, int nteams, const MgLevel *chain,
-                        const VecDev *vs, int burst, unsigned *bars );
+                        const VecDev *vs, int burst, unsigned *bars, unsigned polls, ErrRec *err );
 // mg.cu
 void launch_mg_level0( const Launch &L, const MgLevel *lv, const VecDev *vs, const Chunk *ch, int nch );
 void launch_mg_coarsen( const Launch &L, const MgLevel *lv, int nprob, const Chunk *ch, int nch, ErrRec *err );

@@ -36,7 +36,6 @@ constexpr int PCG_SMEM = 220 * 1024;         // dynamic shared memory of a block
 // the levels of at most this many rows are the first block's: a barrier and the steps' latency cost the team more than a
 // few rounds of the block's warps (1,251 rows: 6,000 cycles by one block, 8,000 with the team's two barriers)
 constexpr int PCG_CHAIN_GRID = 1600, PCG_CHAIN_CLUSTER = 512;
-constexpr unsigned PCG_SPIN = 1u << 21;      // polls of a barrier before it gives up (seconds)
 constexpr float PCG_OMEGA = 0.8f, PCG_ALPHA = 1.5f;      // (the smoother's and the correction's factors of mg.cu)
 
 // rows of a share: a function of the row count alone, at most 148 shares
@@ -48,7 +47,8 @@ __host__ __device__ inline int pcg_share_rows( int n ) {
 struct Team {
     int rank, size;                          // this block in its team
     unsigned *bar;                           // the team's counter; NULL: the team is a cluster
-    int *dead;                               // (shared) set when a wait ran out
+    int *dead;                               // (shared) set when a wait ran out, after `polls` of them
+    unsigned polls;
     unsigned goal;                           // the arrivals that the next barrier waits for
     SDOT_DEV void sync() {
         if ( size == 1 ) { __syncthreads(); return; }
@@ -61,11 +61,11 @@ struct Team {
         if ( threadIdx.x == 0 && ! *dead ) {
             asm volatile( "red.release.gpu.global.add.u32 [%0], 1;" ::"l"( bar ) : "memory" );
             unsigned now = 0, k = 0;
-            for ( ; k < PCG_SPIN; ++k ) {
+            for ( ; k < polls; ++k ) {
                 asm volatile( "ld.acquire.gpu.global.u32 %0, [%1];" : "=r"( now ) : "l"( bar ) : "memory" );
                 if ( int( now - goal ) >= 0 ) break;
             }
-            if ( k == PCG_SPIN ) *dead = 1;
+            if ( k == polls ) *dead = 1;
         }
         __syncthreads();
     }
@@ -415,7 +415,7 @@ struct Pcg {
                 if ( rnorm <= tol * bnorm ) conv = 1;
                 else if ( it >= maxit ) { conv = 2; fail = 1; }
             }
-            if ( *T.dead ) { conv = 2; fail = 1; }      // (a barrier gave up: the system fails, every block leaves)
+            if ( *T.dead ) { conv = 2; fail = 1; }      // (a barrier gave up: every block leaves, and the launch is an error)
             if ( conv != 0 ) break;
             double rz1 = s.y;
             if ( L > 0 ) {
@@ -448,7 +448,7 @@ struct Pcg {
 
 // teams: each block's { problem, rank, team size, team }; bars: a counter per team, zeroed (NULL: the teams are clusters)
 __global__ void __launch_bounds__( PCG_T, 1 ) k_pcg( const PcgProb *__restrict__ probs, const int4 *__restrict__ teams, const MgLevel *__restrict__ chain,
-                                                 const VecDev *__restrict__ vs, int burst, unsigned *bars ) {
+                                                 const VecDev *__restrict__ vs, int burst, unsigned *bars, unsigned polls, ErrRec *err ) {
     extern __shared__ __align__( 16 ) char pcg_smem[];
     __shared__ double2 sh[ PCG_SG * PCG_W ];
     __shared__ SLev lv[ MG_MAX_LEVELS ];
@@ -457,7 +457,7 @@ __global__ void __launch_bounds__( PCG_T, 1 ) k_pcg( const PcgProb *__restrict__
     const PcgProb P = probs[ t.x ];
     const VecDev &V = vs[ P.vec ];
     if ( threadIdx.x == 0 ) dead = 0;
-    Team T{ t.y, t.z, bars ? bars + t.w : nullptr, &dead, 0u };
+    Team T{ t.y, t.z, bars ? bars + t.w : nullptr, &dead, polls, 0u };
     const double done = V.sc[ SC_CONV ];
     __syncthreads();
     T.sync();                                // (read by every block before the first one's last write)
@@ -465,6 +465,8 @@ __global__ void __launch_bounds__( PCG_T, 1 ) k_pcg( const PcgProb *__restrict__
     const int small = bars ? PCG_CHAIN_GRID : PCG_CHAIN_CLUSTER;
     if ( P.count > 0 && chain[ P.first ].pack == 8 ) Pcg<8, 8>::run( V, chain + P.first, P.count, burst, small, T, sh, lv, Smem{ pcg_smem, pcg_smem + PCG_SMEM } );
     else Pcg<4, 4>::run( V, chain + P.first, P.count, burst, small, T, sh, lv, Smem{ pcg_smem, pcg_smem + PCG_SMEM } );
+    // a wait that ran out: the device did not run the team's blocks together -- not a failure of the system
+    if ( threadIdx.x == 0 && dead && atomicCAS( &err->code, 0, 2 ) == 0 ) { err->kind = 0; err->prob = t.x; err->seed = -1; err->needed = 0; }
 }
 
 // the launch of `blocks` blocks, in clusters of `cluster` (0: cooperative)
@@ -559,7 +561,7 @@ void pcg_plan( const std::vector<int> &rows, const PcgDevice &D, std::vector<Pcg
 }
 
 cudaError_t launch_pcg( const Launch &L, const PcgProb *probs, const int4 *teams, int nblocks, int cluster, int nteams, const MgLevel *chain,
-                        const VecDev *vs, int burst, unsigned *bars ) {
+                        const VecDev *vs, int burst, unsigned *bars, unsigned polls, ErrRec *err ) {
     if ( nblocks <= 0 ) return cudaSuccess;
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute at;
@@ -570,7 +572,7 @@ cudaError_t launch_pcg( const Launch &L, const PcgProb *probs, const int4 *teams
         const cudaError_t e = cudaMemsetAsync( bars, 0, size_t( nteams ) * sizeof( unsigned ), L.stream );
         if ( e != cudaSuccess ) return e;
     }
-    const cudaError_t e = cudaLaunchKernelEx( &cfg, k_pcg, probs, teams, chain, vs, burst, bars );
+    const cudaError_t e = cudaLaunchKernelEx( &cfg, k_pcg, probs, teams, chain, vs, burst, bars, polls, err );
     ++*L.launches;
     return e;
 }

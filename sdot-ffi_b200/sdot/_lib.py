@@ -83,6 +83,7 @@ SIGNATURES = {
     "sdot_context_kernel_launches": (ctypes.c_uint64, [_P]),
     "sdot_context_set_timing": (ctypes.c_int32, [_P, ctypes.c_int32]),
     "sdot_context_set_counters": (ctypes.c_int32, [_P, ctypes.c_int32]),
+    "sdot_context_set_barrier_polls": (ctypes.c_int32, [_P, ctypes.c_uint32]),
     "sdot_context_gather_counters": (ctypes.c_int32, [_P, ctypes.c_int32, ctypes.POINTER(ctypes.c_uint64), ctypes.c_int32]),
     "sdot_context_memory": (ctypes.c_int32, [_P, ctypes.POINTER(ctypes.c_uint64), ctypes.POINTER(ctypes.c_uint64),
                                              ctypes.POINTER(ctypes.c_uint64), ctypes.c_int32]),

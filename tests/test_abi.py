@@ -93,6 +93,7 @@ def test_the_counters_and_the_moments_adjoint_refuse_null_arguments():
     L = _lib.load()
     counts = (ctypes.c_uint64 * 5)()
     assert L.sdot_context_set_counters(None, 1) == _lib.SDOT_ERR_ARGS
+    assert L.sdot_context_set_barrier_polls(None, 1) == _lib.SDOT_ERR_ARGS
     assert L.sdot_context_gather_counters(None, 2, counts, 0) == _lib.SDOT_ERR_ARGS
     st = _lib.Status()
     desc = _lib.DiagramDesc()

@@ -9,7 +9,7 @@ import pytest
 import scipy.sparse as sp
 
 from sdot import Box, Iterative, OtProblem, SumOfDiracs, Tuning, _lib
-from sdot.SdotPlanNd import SdotPlanNd
+from sdot.SdotPlanNd import SdotPlanNd, solver_options
 
 pytestmark = pytest.mark.gpu
 
@@ -72,3 +72,36 @@ def test_a_system_has_the_same_bits_in_any_team(d, n, others):
     batch = SdotPlanNd._solve_many(rest[:2] + [one] + rest[2:], settings)[2]
     assert alone.stats["lin_nb_iter"] == batch.stats["lin_nb_iter"]
     assert (alone.weights == batch.weights).all() and (alone.cell_masses == batch.cell_masses).all()
+
+
+def test_a_barrier_that_waits_in_vain_is_an_error():
+    """with a single poll the first blocks of a team give up before the last has come: the call says so -- it is not a system that the
+    CG could not solve --, and the context solves again afterwards"""
+    n = 20011
+    rng = np.random.default_rng(1)
+    pos = rng.uniform(size=(n, 2))
+    problem = (pos, None, None, np.zeros(2), np.ones(2), ("uniform", 1.0))
+    options = solver_options(Iterative(tol=0.0, tuning=Tuning(mass_rtol=1e-8)), n, 2)
+    L = _lib.load()
+    ctx = _lib.new_context()
+    try:
+        before, = _lib.solve_batch([problem], [options], ctx=ctx)
+        assert L.sdot_context_set_barrier_polls(ctx, 1) == _lib.SDOT_OK
+        failed, = _lib.solve_batch([problem], [options], ctx=ctx)
+        assert isinstance(failed, RuntimeError) and "barrier" in str(failed)
+        assert L.sdot_context_set_barrier_polls(ctx, 0) == _lib.SDOT_OK
+        after, = _lib.solve_batch([problem], [options], ctx=ctx)
+        assert (after["weights"] == before["weights"]).all()
+    finally:
+        _lib.destroy_context(ctx)
+    A, dia = ring(n, n)
+    b = rng.normal(size=n)
+    b -= b.mean()
+    L.sdot_context_set_barrier_polls(_lib.context(), 1)
+    try:
+        for method in (0, 1):
+            with pytest.raises(RuntimeError, match="barrier"):
+                _lib.linear_solve(A.indptr, A.indices, A.data, dia, b, tol=1e-9, method=method)
+    finally:
+        L.sdot_context_set_barrier_polls(_lib.context(), 0)
+    assert _lib.linear_solve(A.indptr, A.indices, A.data, dia, b, tol=1e-9)[1][0] > 0
