@@ -1370,16 +1370,11 @@ void launch_cells3d( const Launch &L, const ProbDev *probs, const Chunk *chunks,
                      const Split3 *sp ) {
     if ( nchunks <= 0 ) return;
     const size_t smem = sizeof( Cell3 ) * W3;
-    static bool configured = false;
-    if ( ! configured ) {
-        for ( auto k : { k_cells3d<false>, k_cells3d<true> } ) {
-            cudaFuncSetAttribute( k, cudaFuncAttributeMaxDynamicSharedMemorySize, int( smem ) );
-            cudaFuncSetAttribute( k, cudaFuncAttributePreferredSharedMemoryCarveout, 100 );
-        }
-        configured = true;
-    }
     // the counting instantiation only when the search's reads are counted (F_GATHER): the other compiles without them
     auto *kern = ( flags & F_GATHER ) ? k_cells3d<true> : k_cells3d<false>;
+    // (per device: set for every launch)
+    cudaFuncSetAttribute( kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int( smem ) );
+    cudaFuncSetAttribute( kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100 );
     if ( ! sp ) {
         kern<<<nchunks, 32 * W3, smem, L.stream>>>( probs, chunks, nchunks, flags, err, ovf, 0, Split3{} );
         ++*L.launches;
@@ -1394,11 +1389,7 @@ void launch_cells3d( const Launch &L, const ProbDev *probs, const Chunk *chunks,
 void launch_cells3d_big( const Launch &L, const ProbDev *probs, const OvfList *ovf, int count, unsigned flags, ErrRec *err, OvfList *next ) {
     if ( count <= 0 ) return;
     const size_t smem = sizeof( Cell3B );
-    static bool configured = false;
-    if ( ! configured ) {
-        cudaFuncSetAttribute( k_cells3d_big, cudaFuncAttributeMaxDynamicSharedMemorySize, int( smem ) );
-        configured = true;
-    }
+    cudaFuncSetAttribute( k_cells3d_big, cudaFuncAttributeMaxDynamicSharedMemorySize, int( smem ) );      // (per device)
     k_cells3d_big<<<count < 296 ? count : 296, 32, smem, L.stream>>>( probs, ovf, count, flags, err, next );
     ++*L.launches;
 }

@@ -1643,6 +1643,7 @@ struct VecBatch {
         launch_mg_level0( L, dlv[ 0 ], dv, dbuild0, int( build0.size() ) );
         for ( int l = 0; l + 1 < maxL; ++l ) launch_mg_coarsen( L, dlv[ l ], int( lv[ l ].size() ), dcrs[ l ], int( crs[ l ].size() ), err );
         launch_mg_bottom_build( L, dbottom, int( bottom.size() ) );
+        CK( cudaGetLastError() );              // (a refused launch would leave a hierarchy of whatever its memory held)
     }
     // up to `burst` iterations of a batch of the team CG
     void pcg( Ctx &c, int burst ) {

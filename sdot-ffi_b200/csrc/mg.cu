@@ -405,12 +405,9 @@ void launch_mg_coarsen( const Launch &L, const MgLevel *lv, int nprob, const Chu
     if ( nch <= 0 ) return;
     // the pairs of each warp's coarse row: MG_PAIRS keys (8 bytes) and values (4 bytes)
     constexpr int smem = MG_WARPS * MG_PAIRS * 12;
-    static bool configured = false;
-    if ( ! configured ) {
-        cudaFuncSetAttribute( k_mg_count, cudaFuncAttributeMaxDynamicSharedMemorySize, smem );
-        cudaFuncSetAttribute( k_mg_fill, cudaFuncAttributeMaxDynamicSharedMemorySize, smem );
-        configured = true;
-    }
+    // (past the 48 KB that a launch has by itself, and per device: set for every launch)
+    cudaFuncSetAttribute( k_mg_count, cudaFuncAttributeMaxDynamicSharedMemorySize, smem );
+    cudaFuncSetAttribute( k_mg_fill, cudaFuncAttributeMaxDynamicSharedMemorySize, smem );
     k_mg_count<<<nch, 32 * MG_WARPS, smem, L.stream>>>( lv, ch, nch, err );
     k_mg_scan<<<nprob, 1024, 0, L.stream>>>( lv );
     k_mg_fill<<<nch, 32 * MG_WARPS, smem, L.stream>>>( lv, ch, nch );

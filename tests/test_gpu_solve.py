@@ -420,3 +420,24 @@ def test_the_limits_step_reaches_the_oracle_plan(continuation):
                   density=("image", [0, 0], step, norm.values))
     assert ref["stats"]["status"] == 1
     assert np.abs(plan.weights - ref["weights"]).max() <= 1e-7 * np.abs(ref["weights"]).max()
+
+
+@pytest.mark.parametrize("d", [2, 3])
+def test_a_second_device_of_the_process(d):
+    """what a launch needs set on its device (the shared memory of the hierarchy's build and of the 3D cells) is set on each one"""
+    import torch
+    if torch.cuda.device_count() < 2:
+        pytest.skip("one device")
+    from sdot import _lib
+    from sdot.SdotPlanNd import solver_options
+    pos = np.random.default_rng(d).uniform(size=(3000, d))
+    options = solver_options(Iterative(tol=0.0, tuning=Tuning(mass_rtol=1e-8)), len(pos), d)
+    weights = []
+    for device in (0, 1):
+        ctx = _lib.new_context(device)
+        try:
+            r, = _lib.solve_batch([(pos, None, None, np.zeros(d), np.ones(d), ("uniform", 1.0))], [options], ctx=ctx)
+            weights.append(r["weights"])
+        finally:
+            _lib.destroy_context(ctx)
+    assert (weights[0] == weights[1]).all()
