@@ -1509,6 +1509,7 @@ struct VecBatch {
     std::vector<MgLevel> cchain;
     std::vector<int> crows;
     std::vector<PcgLaunch> groups;
+    double pcg_us = 0;                             // an iteration of them, about
     std::vector<int4> cteams;
     PcgProb *dcprob = nullptr;
     int4 *dcteams = nullptr;
@@ -1607,7 +1608,7 @@ struct VecBatch {
         parts.push_back( { build0.data(), build0.size() * sizeof( Chunk ) } );
         parts.push_back( { cprob.data(), cprob.size() * sizeof( PcgProb ) } );
         parts.push_back( { cchain.data(), cchain.size() * sizeof( MgLevel ) } );
-        if ( ! crows.empty() ) pcg_plan( crows, c.pcg_device(), groups, cteams );
+        if ( ! crows.empty() ) pcg_us = pcg_plan( crows, c.pcg_device(), groups, cteams );
         const std::vector<unsigned> bars( crows.size(), 0u );
         parts.push_back( { cteams.data(), cteams.size() * sizeof( int4 ) } );
         parts.push_back( { bars.data(), bars.size() * sizeof( unsigned ) } );
@@ -1702,7 +1703,7 @@ static void run_burst( Ctx &c, const std::vector<long long> &key, Issue issue ) 
 }
 
 constexpr int MG_BURST_SOLVE = 8;
-constexpr int PCG_BURST = 256;       // iterations of a team CG launch that nothing else waits for (a few ms)
+constexpr int PCG_BURST = 256;       // iterations of a team CG launch that nothing else waits for
 int mg_linear_solve( Ctx &c, const VecDev &V0, long nnz, double *hsc ) {
     SolveJob J;                                      // only its hierarchy is used
     J.G.dim = nnz > 10 * long( V0.n ) ? 3 : 2;       // the aggregates of a 3D Laplacian (about 15 entries a row) pack 8 rows
@@ -2050,8 +2051,8 @@ void jobs_tick( Ctx &c, std::vector<SolveJob *> &jobs ) {
         double rows = 0;
         for ( auto &v : cgc.v ) rows += v.n;
         c.timer.begin( c.stream, K_CG, rows );
-        // the launch ends with the iteration that converges; in a batch it does not hold the others' diagrams up for long
-        cgc.pcg( c, jobs.size() == 1 ? PCG_BURST : ( with_diag.empty() ? PCG_BURST / 4 : PCG_BURST / 8 ) );
+        // the launch ends with the iteration that converges
+        cgc.pcg( c, pcg_burst( cgc.pcg_us, jobs.size() == 1, ! with_diag.empty() ) );
         c.timer.end( c.stream, 1 );
     }
     for ( VecBatch *B : { &cgjx, &cgmx } ) {

@@ -439,9 +439,11 @@ struct PcgDevice { int blocks, clusters[ 5 ]; };
 PcgDevice pcg_device();
 // the launches of the CG of problems of these row counts: the problems [ prob, prob + nprob ), the
 // blocks [ block, block + nblock ) of `teams`, { problem, rank, team size, team } each (counted from `prob`), the cluster size,
-// 0 for a cooperative launch
+// 0 for a cooperative launch.  Returns about how long an iteration of them all takes, us
 struct PcgLaunch { int prob, nprob, block, nblock, cluster; };
-void pcg_plan( const std::vector<int> &rows, const PcgDevice &D, std::vector<PcgLaunch> &launches, std::vector<int4> &teams );
+double pcg_plan( const std::vector<int> &rows, const PcgDevice &D, std::vector<PcgLaunch> &launches, std::vector<int4> &teams );
+// the iterations of a launch, for iterations of `us`: of a solve `alone` in the engine, or with others, some with `diagrams` waiting
+int pcg_burst( double us, bool alone, bool diagrams );
 // up to `burst` iterations of every problem's CG, the start included when its SC_ITER is negative; bars: a counter a problem; a
 // barrier that gives up after `polls` fails its problem and is recorded in `err`
 cudaError_t launch_pcg( const Launch &L, const PcgProb *probs, const int4 *teams, int nblocks, int cluster, int nteams, const MgLevel *chain,

@@ -536,7 +536,7 @@ static int pcg_teams( const int *rows, int np, const PcgDevice &D, std::vector<i
 // us (its barriers and coarse levels; a round's latency; what no longer fits in shared memory).  Measured, ms of CG with so many
 // systems a launch: 65 of 20,011 rows, all 259, 33 199, 16 182, 8 219, 4 320; 17 of 100,003, all 279, 9 255, 4 212, 2 280, 1 435;
 // 33 of 50,003, all 264, 17 237, 8 183, 4 238
-void pcg_plan( const std::vector<int> &rows, const PcgDevice &D, std::vector<PcgLaunch> &launches, std::vector<int4> &teams ) {
+double pcg_plan( const std::vector<int> &rows, const PcgDevice &D, std::vector<PcgLaunch> &launches, std::vector<int4> &teams ) {
     const int np = int( rows.size() );
     launches.clear();
     teams.clear();
@@ -558,6 +558,15 @@ void pcg_plan( const std::vector<int> &rows, const PcgDevice &D, std::vector<Pcg
         }
         if ( least < 0 || time < least ) { least = time; launches = plan; teams = blocks; }
     }
+    return 0.1 * double( least );
+}
+
+// the launches hold the stream until their slowest system has had its burst: 10 ms at most where the solve is alone and a request
+// may come (256 iterations of up to 100,000 rows; 34 of 1e6), 4 ms where other solves wait, and half as many iterations
+// where their diagrams do; not under 8, which a tick's copies and decisions (0.2 ms) cost a tenth of at most
+int pcg_burst( double us, bool alone, bool diagrams ) {
+    const int most = alone ? 256 : ( diagrams ? 32 : 64 );
+    return std::max( 8, std::min( most, int( ( alone ? 10000 : 4000 ) / us ) ) );
 }
 
 cudaError_t launch_pcg( const Launch &L, const PcgProb *probs, const int4 *teams, int nblocks, int cluster, int nteams, const MgLevel *chain,

@@ -20,7 +20,7 @@ namespace sdot {
 #include "teams.inc"
 }
 using namespace sdot;
-// SMs, the clusters of 1, 2, 4, 8 and 16 that run at once, the systems, their rows in; a line per launch: problems, cluster size, then { problem, rank, size, team } a block
+// SMs, the clusters of 1, 2, 4, 8 and 16 that run at once, the systems, their rows in; us an iteration, the bursts, then a line per launch: problems, cluster size, then { problem, rank, size, team } a block
 int main() {
     PcgDevice D;
     int np;
@@ -31,7 +31,8 @@ int main() {
     for ( int &n : rows ) std::cin >> n;
     std::vector<PcgLaunch> launches;
     std::vector<int4> t;
-    pcg_plan( rows, D, launches, t );
+    const double us = pcg_plan( rows, D, launches, t );
+    std::printf( "%.1f %d %d %d\n", us, pcg_burst( us, true, false ), pcg_burst( us, false, false ), pcg_burst( us, false, true ) );
     for ( const PcgLaunch &l : launches ) {
         std::printf( "%d %d", l.nprob, l.cluster );
         for ( int k = l.block; k < l.block + l.nblock; ++k ) std::printf( " %d %d %d %d", t[ k ].x, t[ k ].y, t[ k ].z, t[ k ].w );
@@ -58,9 +59,12 @@ def teams(tmp_path_factory):
     def run(sms, rows):
         given = [sms, *CLUSTERS[sms], len(rows), *rows]
         out = subprocess.run([exe], input=" ".join(map(str, given)), check=True, capture_output=True, text=True).stdout
-        for line in out.splitlines():
+        us, *bursts = out.splitlines()[0].split()
+        launches = []
+        for line in out.splitlines()[1:]:
             nprob, cluster, *v = map(int, line.split())
-            yield nprob, cluster, list(zip(*[iter(v)] * 4))
+            launches.append((nprob, cluster, list(zip(*[iter(v)] * 4))))
+        return launches, float(us), [int(b) for b in bursts]
     return run
 
 
@@ -74,7 +78,7 @@ def shares(n):
                                   [1000000] + [3000] * 100, [4001, 100, 20011, 150]])
 def test_every_system_has_its_blocks(teams, sms, rows):
     at = 0
-    for nprob, cluster, blocks in teams(sms, rows):
+    for nprob, cluster, blocks in teams(sms, rows)[0]:
         assert 1 <= nprob <= len(blocks) <= sms
         assert not cluster or nprob <= CLUSTERS[sms][cluster.bit_length() - 1]
         of = {}
@@ -95,7 +99,17 @@ def test_a_batch_of_large_systems_fills_the_sms(teams, rows):
     """the rows of the fullest block of each launch, together, against the rows an SM has to do at least: a third more at most (the
     clusters of one size left half of the SMs idle)"""
     at = fullest = 0
-    for nprob, _, blocks in teams(148, rows):
+    for nprob, _, blocks in teams(148, rows)[0]:
         fullest += max(-(-rows[at + problem] // size) for problem, _, size, _ in blocks)
         at += nprob
     assert fullest <= 4 / 3 * sum(rows) / 148
+
+
+@pytest.mark.parametrize("rows", [[1000], [20011], [100003], [1000000], [100003] * 9, [20011] * 65, [1000000] + [1000] * 7, [4000000]])
+def test_a_launch_holds_the_stream_for_milliseconds(teams, rows):
+    """10 ms where the solve is alone, 4 where others wait, and 8 iterations at least"""
+    _, us, (alone, others, diagrams) = teams(148, rows)
+    for burst, most, ms in ((alone, 256, 10), (others, 64, 4), (diagrams, 32, 4)):
+        assert 8 <= burst <= most
+        assert burst == 8 or burst * us <= 1000 * ms
+        assert burst == most or (burst + 1) * us > 1000 * ms
