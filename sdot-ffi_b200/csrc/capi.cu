@@ -288,7 +288,7 @@ int32_t sdot_cells( sdot_context ctx, const sdot_diagram_desc *desc, sdot_cells_
         c.timer.begin( c.stream, dim == 2 ? K_CELLS2D : K_CELLS3D, double( n ) );
         launch_wpyr( L, dd.as<ProbDev>(), 1 );
         if ( dim == 2 ) launch_cells2d( L, dd.as<ProbDev>(), ( Chunk * ) ( ( char * ) dd.p + o2 ), int( ch.size() ), flags, c.derr, c.dovf,
-                                        P.fp32 ? 2 : ( P.dkind == D_GAUSS ? 5 : 1 ) );
+                                        clips2d( P ) );
         else launch_cells3d( L, dd.as<ProbDev>(), ( Chunk * ) ( ( char * ) dd.p + o2 ), int( ch.size() ), flags, c.derr, c.dovf, sp );
         c.timer.end( c.stream, sp ? 2 : 1 );
         run_big_cells( c, dd.as<ProbDev>(), flags );
@@ -453,7 +453,7 @@ int32_t sdot_laplacian( sdot_context ctx, const sdot_diagram_desc *desc, int64_t
         CK( cudaMemsetAsync( &c.dovf->count, 0, sizeof( int ), c.stream ) );
         launch_wpyr( L, ( ProbDev * ) base, 1 );
         if ( dim == 2 ) launch_cells2d( L, ( ProbDev * ) base, ( Chunk * ) ( base + o1 ), int( ch.size() ), F_FACETS | F_USER_ORDER, c.derr, c.dovf,
-                                        P.dkind == D_GAUSS ? 5 : 1 );
+                                        clips2d( P ) );
         else
             launch_cells3d( L, ( ProbDev * ) base, ( Chunk * ) ( base + o1 ), int( ch.size() ), F_FACETS | F_USER_ORDER, c.derr, c.dovf,
                             P.dkind == D_GAUSS ? split3_for( c, int( ch.size() ), n ) : nullptr );

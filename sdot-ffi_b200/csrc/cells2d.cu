@@ -868,7 +868,9 @@ __device__ __noinline__ void vjp2( const ProbDev &P, int lane, bool fac, int ui,
 // What bounds a whole cell: code.  The clip's walk and the quadrature with its error functions do not fit the instruction
 // cache together (13 of the 21 cycles between two instructions of a warp went into waiting for it), so the gaussian cells
 // of a diagram with facets are clipped and stored by one pass and integrated by the next: a diagram of 20,011 seeds under
-// 4 gaussians takes 61 ns a cell instead of 96.  Without facets there is no table to store in, and the cells stay whole.
+// 4 gaussians takes 61 ns a cell instead of 96.  A small diagram is one wave of warps whose longest cell bounds it, and pays for
+// the second launch: under GAUSS2_SPLIT cells they stay whole (at a fit's weights, whole / two passes, us: 300 cells 106 / 125,
+// 1,000 122 / 134, 2,000 173 / 171, 3,000 176 / 164, 10,000 588 / 392).  Without facets there is no table to store in, and the cells stay whole.
 //
 // The polygon waits in the cell's own row of the neighbour table, which the second pass then writes, so the passes need no
 // memory of their own: its vertices in the coefficients (16 at most: a row holds CAP2 = 32 of them), its edges' ids in the
@@ -909,7 +911,7 @@ __global__ void __launch_bounds__( 256, 3 ) k_cells2d( const ProbDev *__restrict
         const Chunk ch = chunks[ c ];
         const ProbDev &P = probs[ ch.prob ];
         if ( ( P.fp32 != 0 ) != F32 ) continue;          // (block uniform: the other launch's)
-        const bool two = mode != 0 && P.dkind == D_GAUSS && facets && P.cap >= 2 * MROW2;
+        const bool two = mode != 0 && P.dkind == D_GAUSS && P.n >= GAUSS2_SPLIT && facets && P.cap >= 2 * MROW2;
         if ( mode == 2 && ! two ) continue;
         const bool report = ( flags & F_REPORT ) && ! ( mode == 1 && two );
         double *rep = sh_rep[ warp ];          // this warp's report accumulators (lane 0 updates them)

@@ -1974,7 +1974,7 @@ void jobs_tick( Ctx &c, std::vector<SolveJob *> &jobs ) {
                 c.timer.begin( c.stream, dim == 2 ? K_CELLS2D : K_CELLS3D, seeds );
                 int clips = 0;
                 if ( dim == 2 )
-                    for ( auto &ch : CX[ q ] ) clips |= PX[ ch.prob ].fp32 ? 2 : ( PX[ ch.prob ].dkind == D_GAUSS ? 5 : 1 );
+                    for ( auto &ch : CX[ q ] ) clips |= clips2d( PX[ ch.prob ] );
                 if ( dim == 2 ) launch_cells2d( L, dp, dc, int( CX[ q ].size() ), flags, c.derr, c.dovf, clips );
                 else launch_cells3d( L, dp, dc, int( CX[ q ].size() ), flags, c.derr, c.dovf, sp );
                 c.timer.end( c.stream, sp ? 2 : 1 );

@@ -49,14 +49,15 @@ def test_facets_come_in_the_order_met():
         assert (np.diff(shell) >= 0).all(), (i, shell)
 
 
+@pytest.mark.parametrize("others", [300, 3400])
 @pytest.mark.parametrize("sides", [15, 16, 17, 31, 32, 33, 40])
-def test_gaussian_cells_in_two_passes(sides):
-    """under gaussians the cells of a diagram with facets are stored between two passes up to 16 vertices, done again past them,
-    queued past 32: their masses are the bits of the diagram without facets, and all is the oracle's"""
+def test_gaussian_cells_in_two_passes(sides, others):
+    """under gaussians the cells of a diagram of 2500 seeds and more with facets are stored between two passes up to 16 vertices,
+    done again past them, queued past 32; those of fewer seeds are done whole: their masses are the bits of the diagram without facets, and all is the oracle's"""
     rng = np.random.default_rng(sides)
     t = 2 * np.pi * (np.arange(sides) + 0.1 * rng.uniform(size=sides)) / sides
     ring = 0.5 + 0.2 * np.stack([np.cos(t), np.sin(t)], axis=1)
-    far = rng.uniform(size=(300, 2))
+    far = rng.uniform(size=(others, 2))
     far = far[np.linalg.norm(far - 0.5, axis=1) > 0.28]
     pos = np.concatenate([far[:100], [[0.5, 0.5]], ring, far[100:]])
     c, s = rng.uniform(0.2, 0.8, (3, 2)), rng.uniform(0.1, 0.3, 3)
@@ -80,8 +81,8 @@ def test_the_rest_of_a_row_is_empty(d, n, kind):
         dist = sdot.Image(rng.uniform(0.1, 1.0, size=(16, 16)), frame=[1 / 16, 1 / 16])
     if kind == "ring" and n > 1:                           # a cell of 40 edges (queued) and its neighbours of few
         t = 2 * np.pi * np.arange(40) / 40
-        pos[0], pos[1:41] = 0.5, 0.5 + 0.3 * np.stack([np.cos(t), np.sin(t)], axis=1)
-        pos = pos[:41]
+        pos[0], pos[1:41] = 0.5, 0.5 + 0.2 * np.stack([np.cos(t), np.sin(t)], axis=1)
+        pos = pos[(np.arange(n) < 41) | (np.linalg.norm(pos - 0.5, axis=1) > 0.28)]
     nb, ids, coef, meas = _pd(pos, dist=dist).facets()
     past = np.arange(ids.shape[1]) >= nb[:, None]
     assert (ids[past] == -1).all() and (coef[past] == 0).all() and (meas[past] == 0).all()
