@@ -3,7 +3,7 @@
 // A solve is a state machine (start selection, stages of the width continuation, Newton iterations, trial
 // steps, final moments).  `job_run` / `jobs_tick` advance many solves together: each TICK launches
 //   A. one cell kernel over every solve that needs a diagram (trial weights, start weights, a new stage),
-//   B. up to CG_BURST CG iterations over every solve that is solving its Newton system,
+//   B. a burst of CG iterations over every solve that is solving its Newton system,
 // then reads back every solve's scalars in ONE device->host copy and lets each solve take its decisions
 // (accept or halve the step, switch the residual, converge), and finally launches
 //   D. the Laplacian assembly + rhs + CG start of the solves that begin an iteration, and the trial
@@ -625,7 +625,7 @@ static void alloc_job( Ctx &c, SolveJob &J ) {
     J.ocost = A.take<double>( n );
 }
 
-constexpr int MG_CCH = 16;           // coarse rows per chunk of the coarsening kernels (4 a warp: a small level still spreads)
+constexpr int MG_CCH = 16;           // coarse rows per chunk of the coarsening kernels (one a warp: a small level still spreads)
 constexpr int MG_RCH = 64;           // rows per chunk of the cycle's per-level kernels (one pass of a block)
 
 // the level sizes of the hierarchy of a problem of n seeds; 0 levels when it is too small to need one

@@ -22,8 +22,8 @@
 //
 // Sums: the rows are cut in SHARES by the row count alone, each summed by one block in a fixed tree, and every block folds
 // the shares' sums in another; a block that plays several shares sums each in the same tree (the trees of eight together, so
-// that it does not wait at the end of each: 148 systems of 20,011 rows, a block each, 576 -> 469 ms of CG).  A solve is therefore bitwise the
-// same whatever its team's size -- which follows the batch's load -- and whatever else shares the launch.
+// that it does not wait at the end of each: 148 systems of 20,011 rows, a block each, 576 -> 469 ms of CG).  A solve is
+// therefore bitwise the same whatever its team's size -- which follows the batch's load -- and whatever else shares the launch.
 #include "internal.h"
 #include <algorithm>
 
@@ -71,8 +71,8 @@ struct Team {
     }
 };
 
-// the shares' sums (at most 148) folded: every warp by itself, the same sums in every lane (two: both, else the first)
-SDOT_DEV double2 pcg_fold( const double2 *part, int ns, bool two ) {
+// the shares' sums (at most 148) folded: every warp by itself, the same sums in every lane
+SDOT_DEV double2 pcg_fold( const double2 *part, int ns ) {
     double2 v[ ( PCG_MAX_BLOCKS + 31 ) / 32 ];
     double a = 0, b = 0;
 #pragma unroll
@@ -368,7 +368,7 @@ struct Pcg {
                     pcg_share( pq, 0.0, false, s, s0, s1, part2 + par * ns, sh );
                 }
                 T.sync();
-                const double pq = pcg_fold( part2 + par * ns, ns, false ).x;
+                const double pq = pcg_fold( part2 + par * ns, ns ).x;
                 par ^= 1;
                 if ( ! ( pq > 0 ) ) { conv = 2; fail = 1; break; }
                 alpha = rz / pq;
@@ -402,7 +402,7 @@ struct Pcg {
                 pcg_share( rr, zz, L == 0, s, s0, s1, part2 + par * ns, sh );
             }
             T.sync();
-            const double2 s = pcg_fold( part2 + par * ns, ns, L == 0 );
+            const double2 s = pcg_fold( part2 + par * ns, ns );
             par ^= 1;
             rnorm = sqrt( s.x );
             if ( first ) {
@@ -433,7 +433,7 @@ struct Pcg {
                     pcg_share( zz, 0.0, false, s, s0, s1, part2 + par * ns, sh );
                 }
                 T.sync();
-                rz1 = pcg_fold( part2 + par * ns, ns, false ).x;
+                rz1 = pcg_fold( part2 + par * ns, ns ).x;
                 par ^= 1;
             }
             beta = first ? 0.0 : rz1 / rz;
