@@ -463,10 +463,10 @@ void launch_trial( const Launch &L, const VecDev *v, const Chunk *ch, int nch );
 // cells2d.cu / cells3d.cu
 // the limits of the cells below the floor (one thread a cell; chunks of CHUNK cells over the LimDev array)
 void launch_limits2d( const Launch &L, const LimDev *lims, const Chunk *chunks, int nchunks );
-// clips: bit 0 the problems that clip in FP64, bit 1 those that clip in FP32 (ProbDev.fp32): one launch each; bit 2: some of
-// the former are gaussian, whose diagrams with facets take two passes
-// (GAUSS2_SPLIT: from how many cells on, see cells2d.cu)
+// the cells from which on a gaussian diagram with facets takes two passes (why: cells2d.cu)
 constexpr int GAUSS2_SPLIT = 2500;
+// clips: bit 0 the problems that clip in FP64, bit 1 those that clip in FP32 (ProbDev.fp32): one launch each; bit 2: some of
+// the former take two passes.  Of one problem:
 inline int clips2d( const ProbDev &P ) { return P.fp32 ? 2 : ( P.dkind == D_GAUSS && P.n >= GAUSS2_SPLIT ? 5 : 1 ); }
 void launch_cells2d( const Launch &L, const ProbDev *probs, const Chunk *chunks, int nchunks, unsigned flags, ErrRec *err, OvfList *ovf,
                      int clips = 1 );

@@ -447,8 +447,9 @@ struct Pcg {
 };
 
 // teams: each block's { problem, rank, team size, team }; bars: a counter per team, zeroed (NULL: the teams are clusters)
-__global__ void __launch_bounds__( PCG_T, 1 ) k_pcg( const PcgProb *__restrict__ probs, const int4 *__restrict__ teams, const MgLevel *__restrict__ chain,
-                                                 const VecDev *__restrict__ vs, int burst, unsigned *bars, unsigned polls, ErrRec *err ) {
+__global__ void __launch_bounds__( PCG_T, 1 ) k_pcg( const PcgProb *__restrict__ probs, const int4 *__restrict__ teams,
+                                                 const MgLevel *__restrict__ chain, const VecDev *__restrict__ vs, int burst, unsigned *bars,
+                                                 unsigned polls, ErrRec *err ) {
     extern __shared__ __align__( 16 ) char pcg_smem[];
     __shared__ double2 sh[ PCG_SG * PCG_W ];
     __shared__ SLev lv[ MG_MAX_LEVELS ];
@@ -463,8 +464,9 @@ __global__ void __launch_bounds__( PCG_T, 1 ) k_pcg( const PcgProb *__restrict__
     T.sync();                                // (read by every block before the first one's last write)
     if ( done != 0 ) return;                 // (the whole team)
     const int small = bars ? PCG_CHAIN_GRID : PCG_CHAIN_CLUSTER;
-    if ( P.count > 0 && chain[ P.first ].pack == 8 ) Pcg<8, 8>::run( V, chain + P.first, P.count, burst, small, T, sh, lv, Smem{ pcg_smem, pcg_smem + PCG_SMEM } );
-    else Pcg<4, 4>::run( V, chain + P.first, P.count, burst, small, T, sh, lv, Smem{ pcg_smem, pcg_smem + PCG_SMEM } );
+    const Smem S{ pcg_smem, pcg_smem + PCG_SMEM };
+    if ( P.count > 0 && chain[ P.first ].pack == 8 ) Pcg<8, 8>::run( V, chain + P.first, P.count, burst, small, T, sh, lv, S );
+    else Pcg<4, 4>::run( V, chain + P.first, P.count, burst, small, T, sh, lv, S );
     // a wait that ran out: the device did not run the team's blocks together -- not a failure of the system
     if ( threadIdx.x == 0 && dead && atomicCAS( &err->code, 0, 2 ) == 0 ) { err->kind = 0; err->prob = t.x; err->seed = -1; err->needed = 0; }
 }

@@ -42,7 +42,10 @@ static Seeds tied_seeds( int kind ) {
     double c[ 3 ];
     for ( double &x : c ) x = 0.5 + 0.3 * uniform();
     Seeds s;
-    auto add = [&]( double x, double y, double z ) { s.push_back( { c[ 0 ] + x + jitter * uniform(), c[ 1 ] + y + jitter * uniform(), c[ 2 ] + z + jitter * uniform() } ); };
+    auto add = [&]( double x, double y, double z ) {
+        const double jx = jitter * uniform(), jy = jitter * uniform(), jz = jitter * uniform();
+        s.push_back( { c[ 0 ] + x + jx, c[ 1 ] + y + jy, c[ 2 ] + z + jz } );
+    };
     add( 0, 0, 0 );
     if ( kind < 2 ) {
         for ( int i = -2; i <= 2; ++i ) for ( int j = -2; j <= 2; ++j ) for ( int k = -2; k <= 2; ++k )
@@ -134,7 +137,8 @@ static Wide volume_of_faces( const Seeds &s, Wide R ) {
                 const auto A = poly[ i ], B = poly[ ( i + 1 ) % poly.size() ];
                 const Wide sa = a * A[ 0 ] + b * A[ 1 ] - o, sb = a * B[ 0 ] + b * B[ 1 ] - o;
                 if ( sa <= 0 ) cut.push_back( A );
-                if ( ( sa < 0 && sb > 0 ) || ( sa > 0 && sb < 0 ) ) cut.push_back( { A[ 0 ] + sa / ( sa - sb ) * ( B[ 0 ] - A[ 0 ] ), A[ 1 ] + sa / ( sa - sb ) * ( B[ 1 ] - A[ 1 ] ) } );
+                const Wide t = sa / ( sa - sb );
+                if ( ( sa < 0 && sb > 0 ) || ( sa > 0 && sb < 0 ) ) cut.push_back( { A[ 0 ] + t * ( B[ 0 ] - A[ 0 ] ), A[ 1 ] + t * ( B[ 1 ] - A[ 1 ] ) } );
             }
             poly = cut;
         }

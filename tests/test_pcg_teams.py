@@ -20,7 +20,8 @@ namespace sdot {
 #include "teams.inc"
 }
 using namespace sdot;
-// SMs, the clusters of 1, 2, 4, 8 and 16 that run at once, the systems, their rows in; us an iteration, the bursts, then a line per launch: problems, cluster size, then { problem, rank, size, team } a block
+// in: SMs, the clusters of 1, 2, 4, 8 and 16 that run at once, the systems, their rows
+// out: us an iteration, the bursts; a line per launch: problems, cluster size, then { problem, rank, size, team } a block
 int main() {
     PcgDevice D;
     int np;
@@ -51,10 +52,12 @@ def teams(tmp_path_factory):
         i = src.index(a)
         return src[i:src.index(b, i)] + "\n"
     (d / "teams.inc").write_text(piece("constexpr int PCG_T", "\n") + piece("constexpr int PCG_W", "\n") +
-                                 piece("// rows of a share", "struct Team") + piece("// the blocks of each of `np` problems", "cudaError_t launch_pcg"))
+                                 piece("// rows of a share", "struct Team") +
+                                 piece("// the blocks of each of `np` problems", "cudaError_t launch_pcg"))
     (d / "main.cpp").write_text(MAIN)
     exe = str(d / "teams")
-    subprocess.run(["g++", "-O1", "-std=c++17", "-I", str(d), "-I", HERE, "-I", CSRC, "-I", "/usr/local/cuda/include", str(d / "main.cpp"), "-o", exe], check=True)
+    subprocess.run(["g++", "-O1", "-std=c++17", "-I", str(d), "-I", HERE, "-I", CSRC, "-I", "/usr/local/cuda/include",
+                    str(d / "main.cpp"), "-o", exe], check=True)
 
     def run(sms, rows):
         given = [sms, *CLUSTERS[sms], len(rows), *rows]
